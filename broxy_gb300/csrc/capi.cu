@@ -321,7 +321,8 @@ gm_status gm_voxelize(gm_ctx* ctx, const gm_grid_desc* desc, const float* d_poin
   if (!d_grid || (num_triangles > 0 && (!d_points || !d_triangles)) || num_points < 0 || num_triangles < 0)
     return fail(ctx, GM_ERR_INVALID_ARGUMENT, "gm_voxelize: NULL buffer or negative count");
   if ((s = set_device(ctx)) != GM_OK) return s;
-  if ((s = ensure(ctx, (void**)&ctx->vox, ctx->vox_bytes, gm::voxelize_scratch_bytes(desc->res), "voxelizer scratch")) !=
+  if ((s = ensure(ctx, (void**)&ctx->vox, ctx->vox_bytes, gm::voxelize_scratch_bytes(desc->res, num_triangles),
+                  "voxelizer scratch")) !=
       GM_OK)
     return s;
   GM_CHECK_CUDA(ctx,

@@ -308,7 +308,7 @@ cudaError_t launch_scale_brush(int8_t* R, int n, const float* bbox_min, float ce
 cudaError_t launch_voxelize(const float* P, int64_t nv, const uint32_t* T, int64_t nf, int res,
                             const float* bbox_min, float cell_size, uint8_t* grid, uint8_t* scratch_fine,
                             cudaStream_t st, KernelCounter* kc);
-size_t voxelize_scratch_bytes(int res);
+size_t voxelize_scratch_bytes(int res, int64_t triangles);
 // dir 0: z-words -> packed grid; dir 1: packed grid -> z-words
 cudaError_t launch_layout(int res, const uint32_t* zw, uint8_t* grid, int dir, cudaStream_t st, KernelCounter* kc);
 
