@@ -500,7 +500,7 @@ def run_frame_field(args, ctx, X, R, res, desc):
     ctx.profile(False)
     ff.destroy()
     vox = (2 * res) ** 3
-    return {"field_nodes": qres ** 3, "constraints": 4, "generate_ms": round(gen_ms, 2), "cg_iterations": iters,
+    return {"field_nodes": qres ** 3, "constraints": 4, "generate_ms": round(gen_ms, 2), "solver_rounds": iters,
             "closing_ms": round(close_ms, 3), "closing_gvoxel_s": round(vox / (close_ms * 1e-3) / 1e9, 3),
             "mesh_ms_200_bilateral": round(mesh_ms, 3), "triangles": int(T.shape[0]),
             "kernels_ms": {k: round(v["ms"], 3) for k, v in sorted(prof.items(), key=lambda kv: -kv[1]["ms"])[:8]}}

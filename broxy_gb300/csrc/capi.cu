@@ -1099,7 +1099,7 @@ struct gm_frame_field {
 
 namespace {
 
-constexpr int kMaxHardConstraints = 20;  // max_hc_number_ (GMorpho/FrameField.h, FrameField::FrameField)
+constexpr int kMaxHardConstraints = gm::kFrameFieldMaxPoints;  // max_hc_number_ (GMorpho/FrameField.h, FrameField::FrameField)
 
 // The constraint quaternion (sin(theta/2) v, cos(theta/2)) of a twist:
 // theta = |twist| in float, v = twist scaled by 1.f / theta (left as is when
@@ -1215,7 +1215,7 @@ gm_status gm_frame_field_generate(gm_frame_field* ff, int32_t* iterations, void*
       twist_quat(pt.twist, &rhs[4 * (size_t)c]);
     }
     int it = 0;
-    GM_CHECK_CUDA(ctx, gm::frame_field_solve(ff->gpu, nodes.data(), rhs.data(), n, 1e-10, 400000, &it, st, &ctx->kc),
+    GM_CHECK_CUDA(ctx, gm::frame_field_solve(ff->gpu, nodes.data(), rhs.data(), n, 1e-10, &it, st, &ctx->kc),
                   "gm_frame_field_generate");
     if (iterations) *iterations = it;
   }

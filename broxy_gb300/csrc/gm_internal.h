@@ -173,16 +173,22 @@ struct RotCubeArgs {
 size_t rotcube_scratch_bytes(int res);
 
 // ---- frame field: the biharmonic quaternion system (framefield.cu) ----
+constexpr int kFrameFieldMaxPoints = 20;  // hard constraints of a frame field
+
 struct FrameFieldGpu {
   int res = 0;
   float4* quats = nullptr;  // res^3 (x, y, z, w)
-  double* vecs = nullptr;   // x, r, p, y, Ap: 4 doubles per node each
-  double *x = nullptr, *r = nullptr, *p = nullptr, *y = nullptr, *Ap = nullptr;
+  double *x = nullptr, *r = nullptr, *y = nullptr;  // 4 doubles per node each (one allocation, at x)
   double* part = nullptr;   // block partial sums
-  double* sc = nullptr;     // CG scalars
-  double* h_sc = nullptr;   // pinned copy of the scalars
-  uint8_t* S = nullptr;     // screened (hard-constrained) nodes
-  cudaGraphExec_t graph = nullptr;
+  double *dc = nullptr, *rr = nullptr, *small = nullptr;  // scalars (one allocation, at dc)
+  double* h_rr = nullptr;   // pinned copy of the residual norms
+  // the plan of the direct solve (first solve)
+  bool planned = false;
+  double *cosines = nullptr, *lambda = nullptr;  // cosine matrix and eigenvalues (one allocation)
+  double* g = nullptr;      // G^+ of the squared degrees
+  double sum_deg2 = 0;
+  double* HE = nullptr;     // the constrained nodes' columns, HE_cols per node
+  int HE_cols = 0;
 };
 cudaError_t frame_field_alloc(FrameFieldGpu& f, int res);
 void frame_field_free(FrameFieldGpu& f);
@@ -190,10 +196,11 @@ cudaError_t frame_field_fill(FrameFieldGpu& f, float qx, float qy, float qz, flo
                              KernelCounter* kc);
 // Solves (L^T L + S) q_k = b_k for the four components; nodes[c] / rhs4[4c..]
 // are the constrained nodes (x + res*y + res^2*z) and their quaternions, in
-// the order given (the last one on a node wins).  Stops when every
-// component's residual is <= tol * |b_k| or after max_iters iterations.
+// the order given (the last one on a node wins; at most kFrameFieldMaxPoints
+// distinct nodes).  Refines until every component's residual is <= tol *
+// |b_k| (or a bounded number of rounds); *rounds_out: the solutions taken.
 cudaError_t frame_field_solve(FrameFieldGpu& f, const int64_t* nodes, const float* rhs4, int npts, double tol,
-                              int max_iters, int* iters_out, cudaStream_t st, KernelCounter* kc);
+                              int* rounds_out, cudaStream_t st, KernelCounter* kc);
 cudaError_t launch_rotcube_dilation(const RotCubeArgs& a, cudaStream_t st, KernelCounter* kc);
 // The squared lattice distance field of a cubic grid: per fine voxel p (u16,
 // x-fastest, (2 res)^3), the smallest squared distance from lattice point p

@@ -211,6 +211,28 @@ def test_frame_field_matches_oracle(gm_ctx, qres, npts):
     ff.destroy()
 
 
+@pytest.mark.parametrize("qres,npts", [(2, 1), (2, 8), (3, 20), (5, 4), (7, 5), (16, 20), (17, 3), (18, 13)])
+def test_frame_field_sizes(gm_ctx, qres, npts):
+    """Odd and even lattices from the smallest on (the transforms fold a line
+    in halves and run 16 lines a block), one constraint up to 20, points that
+    share a node and a field solved again after a point changed."""
+    import torch
+    rng = np.random.default_rng(100 * qres + npts)
+    pts = [(tuple(rng.uniform(0.01, 0.99, 3)), tuple(rng.normal(size=3))) for _ in range(npts)]
+    ff = api.FrameField(gm_ctx, (0, 0, 0), (1, 1, 1), qres)
+    for pos, tw in pts:
+        ff.add_point(pos, tw)
+    for again in range(2):
+        ff.generate()
+        got = ff.quats().cpu().numpy()
+        torch.cuda.synchronize()
+        want = F.generate(qres, (0, 0, 0), (1, 1, 1), pts)
+        assert np.abs(got - want).max() <= 1e-5 * np.abs(want).max()
+        pts[0] = (pts[0][0], (0.4, -0.2, 0.9))
+        ff.update_point(0, pts[0][1])
+    ff.destroy()
+
+
 def test_frame_field_same_node_last_wins(gm_ctx):
     """Two constraints on one lattice node: S is set once and b takes the
     later point's quaternion (FrameFieldSparseBiharmonic.cu:353-364,
