@@ -104,6 +104,40 @@ def test_rotcube_large_radius(gm_ctx, uniform):
     assert 0.1 < (want[0] == 0xFF).mean() < 0.99
 
 
+@pytest.mark.parametrize("angle", [0.0, 1e-4, 0.02, 0.049, 0.06, np.pi / 4])
+@pytest.mark.parametrize("uniform", [2, 9, 30])
+def test_rotcube_frames_near_the_axes(gm_ctx, angle, uniform):
+    """Frames along the axes, turned by little and by 45 degrees, the smallest
+    radius and radii whose cube meets the grid's border: the distance field's
+    verdicts and the voxels it leaves to the predicate give the oracle's
+    grids."""
+    res, qres = 32, 3
+    rng = np.random.default_rng(int(1000 * angle) + uniform)
+    axis = rng.normal(size=(qres ** 3, 3)) if angle < 0.5 else np.tile([0.0, 0.0, 1.0], (qres ** 3, 1))
+    axis /= np.linalg.norm(axis, axis=1, keepdims=True)
+    Q = np.concatenate([np.sin(angle / 2) * axis, np.full((qres ** 3, 1), np.cos(angle / 2))], 1).astype(np.float32)
+    X = _grid(res, 9900 + uniform, density=0.002 if uniform < 9 else 0.0002, blocks=1)
+    for mode in (0, 1):
+        got = _run(gm_ctx, res, X, Q, qres, uniform=uniform, mode=mode)
+        want = _oracle(res, X, Q, qres, None, uniform, mode)
+        for g, w, name in zip(got, want, "DSC"):
+            assert np.array_equal(g, w), (name, mode)
+
+
+@pytest.mark.parametrize("zero", ["some", "all"])
+def test_rotcube_degenerate_frames(gm_ctx, zero):
+    """Nodes with a zero quaternion have no frame (the reference's normalize
+    divides zero by zero): those queries keep the tree search."""
+    res, qres = 16, 4
+    Q = _field(qres, 9950)
+    Q[::5 if zero == "some" else 1] = 0
+    X = _grid(res, 9960, density=0.003, blocks=1)
+    got = _run(gm_ctx, res, X, Q, qres, uniform=3)
+    want = _oracle(res, X, Q, qres, None, 3, 0)
+    for g, w, name in zip(got, want, "DSC"):
+        assert np.array_equal(g, w), name
+
+
 @pytest.mark.parametrize("res,uniform", [(16, 3), (64, 75)])
 def test_rotcube_smallest_grid_and_huge_radius(gm_ctx, res, uniform):
     """res 16 (four pyramid levels); and radius 75 around one corner block:
