@@ -15,7 +15,6 @@
 
 #include "../../include/gmorpho_gb300.h"
 #include "gm_common.cuh"
-#include "tma.cuh"
 #include "gm_internal.h"
 
 namespace gm {
@@ -221,7 +220,6 @@ gm_status gm_ctx_create(int device, gm_ctx** out) {
   if (cudaSetDevice(device) != cudaSuccess) { delete c; return GM_ERR_CUDA; }
   cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, device);
   if (cudaMalloc(&c->d_int, 16 * sizeof(int)) != cudaSuccess) { delete c; return GM_ERR_OUT_OF_MEMORY; }
-  gm::tma_init();
   *out = c;
   return GM_OK;
 }

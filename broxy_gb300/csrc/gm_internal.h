@@ -40,7 +40,8 @@ struct KernelCounter {
 cudaError_t ensure_dynamic_smem(const void* kernel, size_t bytes);
 
 // The error bits kernels of this library recorded on the current device
-// (kErrTmaTimeout: a TMA tile wait ran out of polls), cleared when `clear`.
+// (kernels with a bounded wait record one; none waits at present), cleared
+// when `clear`.
 cudaError_t kernel_error_flags(unsigned int* flags, bool clear);
 
 // JSON {"name": {"launches": n, "ms": t}, ...} of the counter's totals;

@@ -22,7 +22,6 @@
 // refinement of contour cells only) is then applied exactly by the select
 // kernels, which reproduces the reference grids bit for bit (GM_REF), or
 // skipped (GM_EXACT).
-#include <cudaTypedefs.h>
 #include <string.h>
 
 #include <algorithm>
@@ -31,12 +30,11 @@
 
 #include "gm_common.cuh"
 #include "gm_internal.h"
-#include "tma.cuh"
 
 namespace gm {
 
-// Error bits recorded by kernels (kErrTmaTimeout, ...); read and cleared by
-// kernel_error_flags().
+// Error bits that kernels with a bounded wait record instead of trapping
+// (none waits at present); read and cleared by kernel_error_flags().
 __device__ unsigned int g_kernel_errors = 0;
 
 // A radius field read in place: element (x, y, z) at p[x + y sy + z sz]
@@ -806,22 +804,26 @@ __device__ __forceinline__ uint32_t step_min(uint32_t row, uint32_t g, uint32_t 
   return __viaddmin_u16x2(row, g, best);
 }
 
-template <int G, typename TIn>
-__device__ __forceinline__ uint32_t load_pair(const TIn* p, uint32_t capp) {
-  uint32_t v;
-  if (sizeof(TIn) == 1) {
-    const uint32_t w = *reinterpret_cast<const uint16_t*>(p);
-    const uint32_t a = w & 0xffu, b = w >> 8;
-    v = G != KERN_CUBE ? (a * a) | ((b * b) << 16) : a | (b << 16);
-  } else {
-    v = *reinterpret_cast<const uint32_t*>(p);
-  }
-  return __vminu2(v, capp);  // both lanes saturated at cap
+// Four packed words (8 columns) of a u16 field.
+__device__ __forceinline__ uint4 clamp4(uint4 v, uint32_t capp) {
+  return make_uint4(__vminu2(v.x, capp), __vminu2(v.y, capp), __vminu2(v.z, capp), __vminu2(v.w, capp));
+}
+__device__ __forceinline__ uint32_t min4(uint4 v, uint32_t m) {
+  return __vimin3_u16x2(__vimin3_u16x2(v.x, v.y, m), v.z, v.w);
+}
+// Two u8 distances (the low bytes of a word's halves) as packed u16: squared
+// for the ball, themselves for the cube.
+template <int G>
+__device__ __forceinline__ uint32_t widen_pair(uint32_t w, uint32_t sel) {
+  const uint32_t p = __byte_perm(w, 0u, sel);  // the two bytes, zero-extended
+  if (G == KERN_CUBE) return p;
+  const uint32_t hi = p >> 16;
+  return (p & 0xffffu) * (p & 0xffffu) + (p & 0xffff0000u) * hi;
 }
 
 size_t dpx_smem_bytes(int sub, int halo) {
   const int span = (sub ? 2 * kDpxOut - 1 : kDpxOut) + 2 * halo;
-  return (size_t)2 * span * 32 * sizeof(uint32_t) + 128;  // + slack to align the tile to 128 bytes (TMA)
+  return (size_t)2 * span * 32 * sizeof(uint32_t);
 }
 
 // Where a pass's outputs are needed: tiles whose cells, grown by (gx, ga,
@@ -858,62 +860,77 @@ __device__ bool tile_needed(const NeedMap& nm, int axis, int sub, int o0, int no
   const int lo[3] = {cx0 - nm.gx, (axis == 1 ? ca0 - nm.ga : ct0 - nm.gt), (axis == 1 ? ct0 - nm.gt : ca0 - nm.ga)};
   const int hi[3] = {cx1 + nm.gx, (axis == 1 ? ca1 + nm.ga : ct1 + nm.gt), (axis == 1 ? ct1 + nm.gt : ca1 + nm.ga)};
   const int md[3] = {nm.mdx, nm.mdy, nm.mdz};
-  int a[3], b[3], c[3];
+  int a[3], b[3];
   for (int k = 0; k < 3; k++) {
     a[k] = max(lo[k], 0) >> 3;
     b[k] = min(hi[k] >> 3, md[k] - 1);
-    c[k] = b[k] - a[k] + 1;
   }
-  int any = 0;
-  if (c[0] > 0 && c[1] > 0 && c[2] > 0)
-    for (int i = threadIdx.x; i < c[0] * c[1] * c[2]; i += blockDim.x) {
-      const int ix = a[0] + i % c[0], iy = a[1] + (i / c[0]) % c[1], iz = a[2] + i / (c[0] * c[1]);
-      any |= nm.dmap[idx3(ix, iy, iz, nm.mdx, nm.mdy)];
-    }
-  return __syncthreads_or(any) != 0;
+  // eight blocks along x, four along y a step of the warp
+  const int lane = threadIdx.x & 31;
+  for (int z = a[2]; z <= b[2]; z++)
+    for (int y = a[1] + (lane >> 3); y - (lane >> 3) <= b[1]; y += 4)
+      for (int x = a[0] + (lane & 7); x - (lane & 7) <= b[0]; x += 8) {
+        const bool any = x <= b[0] && y <= b[1] && nm.dmap[idx3(x, y, z, nm.mdx, nm.mdy)] != 0;
+        if (__any_sync(0xffffffffu, any)) return true;
+      }
+  return false;
 }
 
 // Radius bound of one tile of a dilation pass, from the map of the largest
 // raw radius per 16^3 fine voxels: over the tile's x columns and outputs,
 // and its two third-axis coordinates widened by `rext` (the y pass feeds z
-// outputs up to a halo away).  Block-uniform.
+// outputs up to a halo away).  Every warp finds it for itself (4 x 4 map
+// cells across the tile and two along the third axis a step): no barrier.
 __device__ int tile_radius(const uint8_t* __restrict__ rmap, int mbx, int mby, int nx, int n3, int axis, int nout,
                            int o0, int rext, int bx, int bz) {
-  __shared__ int rt_s;
-  if (threadIdx.x == 0) rt_s = 0;
-  __syncthreads();
-  const int xa = (bx * kDpxCols) >> 4, xb = (min(bx * kDpxCols + kDpxCols, nx) - 1) >> 4;
-  const int aa = o0 >> 4, ab = (min(o0 + kDpxOut, nout) - 1) >> 4;
+  const int lane = threadIdx.x & 31;
+  const int ix = ((bx * kDpxCols) >> 4) + (lane & 3), ia = (o0 >> 4) + ((lane >> 2) & 3);
   const int ta = max(2 * bz - rext, 0) >> 4, tb = min(2 * bz + 1 + rext, n3 - 1) >> 4;
-  const int cx = xb - xa + 1, ca = ab - aa + 1, ct = tb - ta + 1;
   int m = 0;
-  for (int i = threadIdx.x; i < cx * ca * ct; i += blockDim.x) {
-    const int ix = xa + i % cx, ia = aa + (i / cx) % ca, it = ta + i / (cx * ca);
-    const int my = axis == 1 ? ia : it, mz = axis == 1 ? it : ia;
-    const int v = rmap[idx3(ix, my, mz, mbx, mby)];
-    m = v > m ? v : m;
-  }
-  for (int o = 16; o > 0; o >>= 1) { const int t = __shfl_xor_sync(0xffffffffu, m, o); m = t > m ? t : m; }
-  if ((threadIdx.x & 31) == 0 && m > 0) atomicMax(&rt_s, m);
-  __syncthreads();
-  return clamp_radius(rt_s);
+  if (16 * ix < nx && 16 * ia < nout)
+    for (int it = ta + (lane >> 4); it <= tb; it += 2) {
+      const int v = rmap[idx3(ix, axis == 1 ? ia : it, axis == 1 ? it : ia, mbx, mby)];
+      m = v > m ? v : m;
+    }
+  return clamp_radius(__reduce_max_sync(0xffffffffu, m));
+}
+
+// First tap k at which the kernel alone reaches d (the -side of LAT lags by
+// one tap and ends with it).
+template <int G>
+__device__ __forceinline__ int last_tap(uint32_t d) {
+  if (G == KERN_CUBE) return (int)d;
+  const float s = __fsqrt_rn((float)d);
+  if (G == KERN_LAT) return (int)ceilf(s);
+  if (G == KERN_CEN2) return (int)ceilf(0.5f * (s + 1.f));
+  return (int)ceilf(0.5f * s) + 1;  // KERN_LAT2
 }
 
 // One tile of a min-plus pass: 64 columns x 64 outputs x 2 third-axis
 // slices, at tile coordinates (bx, by, bz) along (x, outputs, slice pairs),
 // the need map's out0 / third0 offsets included.  The whole block works on
-// it.  With use_tma, the u16 input tile is staged by TMA (tmap: boxes of 64
-// columns x span rows x 1 slice along (x, pass axis, third axis), one per
-// slice; rows are 128 bytes, so each slice starts 128-byte aligned).
+// it.  The taps are at most a third of what a tile costs, so the rest is
+// kept short: 16-byte loads (a thread: 8 or 16 columns of a row, every 16th
+// or 32nd row of its slice), window ends by a square root, the radius bound
+// and the need test per warp without barriers, thresholds as packed adds
+// whose sign bits collect in one word.  Warps whose 16 outputs lie past the
+// field skip the taps (extents are multiples of 16).  Against row-wise
+// 4-byte loads or a TMA box re-read for its minimum, a search loop for the
+// window's end, two walks over the maps with divisions and barriers, and a
+// packing of its own per output: dilation z at 512^3, radius 12, 2017 -> 851
+// instructions a warp's 16 rows (the taps are 448) and 0.287 -> 0.152 ms;
+// the six passes at 1024^3 with a radius field 9.6 -> 6.4 ms.  Bound by the
+// ALU pipe (70-74% busy) and, at the start of a tile, by its loads; sums on
+// the FMA pipe with three-input minima instead of add-mins, three blocks an
+// SM instead of four and an exit test every fourth tap were no faster.
 template <int G, typename TIn, int FIN>
 __device__ __forceinline__ void dpx_tile(const TIn* __restrict__ in, uint16_t* __restrict__ out16,
                                          uint8_t* __restrict__ out8, int nx, int ny, int nz, int axis, int sub,
                                          int halo, uint32_t cap, RField R, int uniform_r, int rx, int ry,
-                                         const uint8_t* __restrict__ rmap, int rext, const NeedMap& need,
-                                         const CUtensorMap* tmap, int use_tma, int bx, int by, int bz) {
-  extern __shared__ uint32_t tile_raw[];
-  uint32_t* tileu = reinterpret_cast<uint32_t*>((reinterpret_cast<uintptr_t>(tile_raw) + 127) & ~(uintptr_t)127);
-  __shared__ uint64_t tma_bar;
+                                         const uint8_t* __restrict__ rmap, int rext, const NeedMap& need, int bx,
+                                         int by, int bz) {
+  extern __shared__ uint4 tile_raw[];
+  uint32_t* tileu = reinterpret_cast<uint32_t*>(tile_raw);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int tpar = w >> 2, grp = w & 3;
   const int x = bx * kDpxCols + 2 * lane;
@@ -924,14 +941,13 @@ __device__ __forceinline__ void dpx_tile(const TIn* __restrict__ in, uint16_t* _
   const int64_t sa = axis == 1 ? (int64_t)nx : (int64_t)nx * ny;
   const int64_t s3 = axis == 1 ? (int64_t)nx * ny : (int64_t)nx;
   const int o0 = by * kDpxOut;
-  const int step = sub ? 2 : 1;
   const int lo = (sub ? 2 * o0 + 1 : o0) - halo;
   const int span = (sub ? 2 * kDpxOut - 1 : kDpxOut) + 2 * halo;
   // Dilation passes with a radius field use the tile's own radius bound:
   // a smaller window (halo_e) and saturation value (cap_e).  Every output
   // that reads this tile has r(p) <= rt, so terms >= (rt+1)^2 never decide.
   int halo_e = halo;
-  if (rmap != nullptr && step == 1) {
+  if (rmap != nullptr && !sub) {
     const int rt = tile_radius(rmap, nx >> 4, ny >> 4, nx, n3, axis, nout, o0, rext, bx, bz);
     const uint32_t ct = G == KERN_CUBE ? (uint32_t)(rt + 1) : (uint32_t)((rt + 1) * (rt + 1));
     cap = ct < cap ? ct : cap;
@@ -943,76 +959,65 @@ __device__ __forceinline__ void dpx_tile(const TIn* __restrict__ in, uint16_t* _
   const bool needed = tile_needed(need, axis, sub, o0, nout, bx, bz);
   const int skip = needed ? halo - halo_e : span;  // tile rows never read
   const uint32_t capp = cap | (cap << 16);
-  const int tile_rows = span;
-  uint32_t* tile = tileu + tpar * tile_rows * 32;
+  uint32_t* tile = tileu + tpar * span * 32;
   const bool colok = x < nx && third < n3;
-  int finite = 0;
-  constexpr bool kTileMin = G == KERN_CEN2 || G == KERN_LAT2 || (G == KERN_LAT && FIN == 1);
-  uint32_t vmin = 0xffffffffu;  // smallest loaded value (both lanes)
-  // TMA staging (u16 inputs): the whole span of both slices, one copy per
-  // slice issued by one thread; rows past the field come back as zeros and
-  // are set to the saturation value below, with the rows [skip, span - skip)
-  // that the taps read.
-  const int nchunks = sizeof(TIn) == 2 && use_tma && span - 2 * skip > 0 ? 1 : 0;  // block-uniform
-  if (nchunks > 0) {
-    if (threadIdx.x == 0) {
-      tma_prefetch_map(tmap);
-      mbar_init(&tma_bar, 1);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      mbar_arrive_expect_tx(&tma_bar, (uint32_t)(2 * span * kDpxCols * sizeof(uint16_t)));
-      const int x0 = bx * kDpxCols, t0 = 2 * bz;
-      for (int tp = 0; tp < 2; tp++) {
-        uint32_t* dst = tileu + tp * tile_rows * 32;
-        if (axis == 1)
-          tma_load_3d(dst, tmap, x0, lo, t0 + tp, &tma_bar);
-        else
-          tma_load_3d(dst, tmap, x0, t0 + tp, lo, &tma_bar);
+  __shared__ uint32_t warp_min[8];
+  {
+    uint32_t vmin = capp;  // smallest loaded value (both lanes)
+    const bool slice = third < n3;
+    if (sizeof(TIn) == 1) {
+      const int c = threadIdx.x & 3, x0 = bx * kDpxCols + 16 * c;
+      const TIn* src = in + x0 + s3 * third;
+      const bool ok = slice && x0 < nx;
+#pragma unroll 2
+      for (int s = skip + ((threadIdx.x & 127) >> 2); s < span - skip; s += 32) {
+        const int p = lo + s;
+        uint4 v0 = make_uint4(capp, capp, capp, capp), v1 = v0;
+        if (ok && p >= 0 && p < na) {
+          const uint4 q = *reinterpret_cast<const uint4*>(src + sa * p);
+          v0 = clamp4(make_uint4(widen_pair<G>(q.x, 0x4140u), widen_pair<G>(q.x, 0x4342u), widen_pair<G>(q.y, 0x4140u),
+                                 widen_pair<G>(q.y, 0x4342u)), capp);
+          v1 = clamp4(make_uint4(widen_pair<G>(q.z, 0x4140u), widen_pair<G>(q.z, 0x4342u), widen_pair<G>(q.w, 0x4140u),
+                                 widen_pair<G>(q.w, 0x4342u)), capp);
+        }
+        uint4* dst = reinterpret_cast<uint4*>(tile + s * 32 + 8 * c);
+        dst[0] = v0;
+        dst[1] = v1;
+        vmin = min4(v1, min4(v0, vmin));
+      }
+    } else {
+      const int c = threadIdx.x & 7, x0 = bx * kDpxCols + 8 * c;
+      const TIn* src = in + x0 + s3 * third;
+      const bool ok = slice && x0 < nx;
+#pragma unroll 4
+      for (int s = skip + ((threadIdx.x & 127) >> 3); s < span - skip; s += 16) {
+        const int p = lo + s;
+        uint4 v = make_uint4(capp, capp, capp, capp);
+        if (ok && p >= 0 && p < na) v = clamp4(*reinterpret_cast<const uint4*>(src + sa * p), capp);
+        *reinterpret_cast<uint4*>(tile + s * 32 + 4 * c) = v;
+        vmin = min4(v, vmin);
       }
     }
-    if (!mbar_wait_bounded(&tma_bar, 0, 1u << 22)) atomicOr(&g_kernel_errors, kErrTmaTimeout);
-  }
-  for (int s = skip + grp; s < span - skip; s += 4) {
-    const int a = lo + s;
-    uint32_t v = capp;
-    if (colok && a >= 0 && a < na)
-      v = nchunks > 0 ? __vminu2(tile[s * 32 + lane], capp) : load_pair<G, TIn>(in + x + sa * a + s3 * third, capp);
-    tile[s * 32 + lane] = v;
-    finite |= v != capp;
-    if (kTileMin) vmin = __vminu2(vmin, v);
-  }
-  __shared__ uint32_t warp_min[8];
-  if (kTileMin) {
-    const uint32_t m2 = (vmin & 0xffffu) < (vmin >> 16) ? (vmin & 0xffffu) : (vmin >> 16);
-    const uint32_t mw = __reduce_min_sync(0xffffffffu, m2);
+    const uint32_t mw = __reduce_min_sync(0xffffffffu, min(vmin & 0xffffu, vmin >> 16));
     if (lane == 0) warp_min[w] = mw;
   }
-  finite = __syncthreads_or(finite);
+  __syncthreads();
   // Every tile value is >= tmin, so a tap whose kernel value reaches
   // cap - tmin cannot bring an output below the saturation value cap: the
   // window of this tile ends at the last tap below it (kernels grow with
   // |delta|).  Erosion passes: their inputs carry the per-site offset
   // K - 4 (r - 1)^2, so tiles whose sites all have small radii need short
-  // windows; the final dilation pass: tiles whose inputs are all far from
-  // the input stop early.  (The first dilation pass, whose tiles next to a
-  // surface hold zeros, is faster without it.)
-  uint32_t tmin = 0;
-  int halo_t = step == 1 ? halo_e : halo;
-  if (kTileMin) {
-    tmin = warp_min[0];
+  // windows; dilation passes: tiles whose inputs are all far from the input
+  // stop early.
+  uint32_t tmin = warp_min[0];
 #pragma unroll
-    for (int i = 1; i < 8; i++) tmin = warp_min[i] < tmin ? warp_min[i] : tmin;
-  }
-  if (kTileMin && finite) {
-    int hm = 1;
-    while (hm < halo_t && (step == 1 ? kern_pos<G>(hm)
-                                     : (kern_g<G>(hm) < kern_g<G>(-hm) ? kern_g<G>(hm) : kern_g<G>(-hm))) +
-                                  tmin < cap)
-      hm++;
-    halo_t = hm < halo_t ? hm : halo_t;
-  }
+  for (int i = 1; i < 8; i++) tmin = min(tmin, warp_min[i]);
   const int obase = o0 + grp * kDpxPer;
+  const bool finite = needed && tmin < cap && obase < nout;  // else every output keeps cap
+  // (the cube combines by the larger of value and kernel: its window ends
+  // with the kernel alone)
+  if (G == KERN_CUBE) tmin = 0;
+  const int halo_t = min(halo_e, max(last_tap<G>(cap - tmin), 1));
   const int sp0 = (sub ? 2 * obase + 1 : obase) - lo;
   uint32_t best[kDpxPer];
   // The lattice-point erosion (KERN_LAT2) is the only pass with outputs at
@@ -1057,10 +1062,11 @@ __device__ __forceinline__ void dpx_tile(const TIn* __restrict__ in, uint16_t* _
         // sp0 + k and sp0 + 15 - k are free now (k < halo_e keeps both in the window)
         wp[u] = tcol[(sp0 + k + kDpxPer) * 32];
         wm[(kDpxPer - 1 - u) % kDpxPer] = tcol[(sp0 - k - 1) * 32];
-        if ((u & 3) == 3) {  // every fourth tap: leave once no output can improve
+        if ((u & 7) == 3) {  // every eighth tap: leave once no output can improve
           uint32_t m = best[0];
 #pragma unroll
-          for (int j = 1; j < kDpxPer; j++) m = __vmaxu2(m, best[j]);
+          for (int j = 1; j + 1 < kDpxPer; j += 2) m = __vimax3_u16x2(m, best[j], best[j + 1]);
+          m = __vmaxu2(m, best[kDpxPer - 1]);
           const uint32_t mx = (m & 0xffffu) > (m >> 16) ? (m & 0xffffu) : (m >> 16);
           // smallest kernel value of the taps to come (k + 1 on either side)
           const uint32_t nxt = G == KERN_CEN2 ? kern_pos<G>(k + 1) : graw;
@@ -1118,10 +1124,11 @@ __device__ __forceinline__ void dpx_tile(const TIn* __restrict__ in, uint16_t* _
           // that R(k) and R(15 - k) leave
           if (k < kp) wp[u] = tb[(k + kDpxPer) * 64];
           if (k < km) wm[(kDpxPer - 1 - u) % kDpxPer] = tb[(-k - 1) * 64];
-          if ((u & 3) == 3) {  // every fourth tap: leave once no output can improve
+          if ((u & 7) == 3) {  // every eighth tap: leave once no output can improve
             uint32_t m = best[0];
 #pragma unroll
-            for (int j = 1; j < kDpxPer; j++) m = __vmaxu2(m, best[j]);
+            for (int j = 1; j + 1 < kDpxPer; j += 2) m = __vimax3_u16x2(m, best[j], best[j + 1]);
+            m = __vmaxu2(m, best[kDpxPer - 1]);
             const uint32_t mx = (m & 0xffffu) > (m >> 16) ? (m & 0xffffu) : (m >> 16);
             const uint32_t np = k + 1 <= kp ? kern_g<G>(2 * (k + 1) + e0) : 0xffffu;
             const uint32_t nm = k + 1 <= km ? kern_g<G>(-2 * (k + 1) + e0) : 0xffffu;
@@ -1137,77 +1144,93 @@ __device__ __forceinline__ void dpx_tile(const TIn* __restrict__ in, uint16_t* _
     for (int j = 0; j < kDpxPer; j++) best[j] = capp;
   }
   if (FIN == 0) {
-    if (!colok) return;
+    if (!colok || obase >= nout) return;
     const int64_t osa = axis == 1 ? (int64_t)nx : (int64_t)nx * ny;
     const int64_t os3 = axis == 1 ? (int64_t)nx * nout : (int64_t)nx;
+    uint16_t* dst = out16 + x + osa * obase + os3 * third;
 #pragma unroll
-    for (int j = 0; j < kDpxPer; j++) {
-      const int o = obase + j;
-      if (o < nout) *reinterpret_cast<uint32_t*>(out16 + x + osa * o + os3 * third) = best[j];
-    }
+    for (int j = 0; j < kDpxPer; j++) *reinterpret_cast<uint32_t*>(dst + osa * j) = best[j];
   } else if (FIN == 3) {
-    if (!colok) return;
+    if (!colok || obase >= nout) return;
     // x is a cell index here; outputs are cells (x, third, o)
+    uint8_t* dst = out8 + idx3(x, third, obase, rx, ry);
+    const uint32_t t1 = 0x80008000u - capp;
 #pragma unroll
     for (int j = 0; j < kDpxPer; j++) {
-      const int o = obase + j;
-      if (o >= nout) continue;
-      const uint32_t v = best[j];
-      uint8_t* dst = out8 + idx3(x, third, o, rx, ry);
-      dst[0] = (v & 0xffffu) < cap ? 1 : 0;
-      dst[1] = (v >> 16) < cap ? 1 : 0;
+      const uint32_t f = ~(best[j] + t1);  // bit 15 of a half: value < cap
+      *reinterpret_cast<uint16_t*>(dst + (int64_t)rx * ry * j) = (uint16_t)(((f >> 15) & 1u) | ((f >> 23) & 0x100u));
     }
   } else {
-    // threshold then pack 2 (x) x 2 (y = third pair) x 2 (z) bits per byte
+    // threshold then pack 2 (x) x 2 (y = third pair) x 2 (z) bits per byte.
+    // value < T exactly when bit 15 of value + 0x8000 - T is clear (both at
+    // most 0x7fff); the 16 outputs' bits collect in one word, the lower
+    // column's in its lower half.
     __shared__ uint32_t xch[4][32][2];
-    const int N = nz;  // fine extent along the pass axis (z)
-    const int ru = clamp_radius(uniform_r);
-    uint32_t bytes[2] = {0u, 0u};  // 8 z pairs: bytes q = 0..7
-#pragma unroll
-    for (int j = 0; j < kDpxPer; j++) {
-      const int z = obase + j;
-      const uint32_t v = best[j];
-      // per-lane thresholds T (bit = value < T)
-      uint32_t tpair;
+    uint32_t acc = 0xffffffffu;  // bit j of a half: output j is not below its threshold
+    if (colok && obase < nout) {
+      const bool field = FIN == 1 && R.p != nullptr;
+      const int8_t* rp = nullptr;
+      uint32_t t1;
       if (FIN == 1) {
-        uint32_t r2;  // the two clamped radii, one per u16 lane
-        if (R.p != nullptr && colok && z < N) {
-          // x even and even strides: a 2-byte aligned pair
-          const uint32_t rr = *reinterpret_cast<const uint16_t*>(R.p + (int64_t)x + third * R.sy + z * R.sz);
-          const uint32_t c = __vmins4(__vmaxs4(rr, 0x02020202u), 0x7f7f7f7fu);  // clamp to [2, 127] per byte
-          r2 = __byte_perm(c, 0u, 0x4140);
-        } else {
-          r2 = (uint32_t)ru | ((uint32_t)ru << 16);
-        }
-        const uint32_t r1 = r2 + 0x00010001u;  // r + 1 per lane (<= 128)
-        if (G == KERN_CUBE) {
-          tpair = r1;  // value <= r
-        } else {
-          const uint32_t lo = r1 & 0xffffu, hi = r1 >> 16;
-          tpair = (lo * lo) | ((hi * hi) << 16);  // value < (r + 1)^2
+        const uint32_t r1 = (uint32_t)clamp_radius(uniform_r) + 1u, t = G == KERN_CUBE ? r1 : r1 * r1;
+        t1 = 0x80008000u - (t | (t << 16));
+        if (field) rp = R.p + (int64_t)x + third * R.sy + obase * R.sz;
+      } else {
+        t1 = 0x80008000u - capp;
+      }
+      if (field) {
+#pragma unroll
+        for (int j = 0; j < kDpxPer; j++) {
+          // x even and even strides: a 2-byte aligned pair of radii,
+          // sign-extended to the halves, at least 2 (at most 127 as bytes)
+          const uint32_t rr = *reinterpret_cast<const uint16_t*>(rp + j * R.sz);
+          uint32_t r2;
+          asm("prmt.b32 %0, %1, 0, 0x9180;" : "=r"(r2) : "r"(rr));
+          const uint32_t r1 = __vmaxs2(r2, 0x00020002u) + 0x00010001u;  // r + 1 (<= 128)
+          uint32_t e = best[j] + 0x80008000u;
+          if (G == KERN_CUBE) {
+            e -= r1;  // value <= r
+          } else {
+            const uint32_t a = r1 & 0xffffu, b = r1 >> 16;
+            e = e - a * a - (r1 & 0xffff0000u) * b;  // value < (r + 1)^2
+          }
+          acc = ((acc >> 1) & 0x7fff7fffu) | (e & 0x80008000u);
         }
       } else {
-        tpair = capp;
+#pragma unroll
+        for (int j = 0; j < kDpxPer; j++) acc = ((acc >> 1) & 0x7fff7fffu) | ((best[j] + t1) & 0x80008000u);
       }
-      const uint32_t m = __vcmpltu2(v, tpair);  // 0xffff per lane below its threshold
-      const uint32_t b2 = (m & 1u) | ((m >> 15) & 2u);
-      const int q = j >> 1, zb = j & 1;
-      bytes[q >> 2] |= (b2 << (2 * tpar + 4 * zb)) << (8 * (q & 3));
+    }
+    // bits of z pair q to byte q: z even to bits 0, 1, z odd to bits 4, 5
+    uint32_t bytes[2];
+    {
+      const uint32_t f = ~acc, u = f & 0xffffu, v = f >> 16;  // the two columns
+      const uint32_t e = (u & 0x5555u) | ((v & 0x5555u) << 1), o = ((u >> 1) & 0x5555u) | (v & 0xaaaau);
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        uint32_t p = ((e >> (8 * h)) & 0xffu) | (((o >> (8 * h)) & 0xffu) << 16);  // four 2-bit fields of each
+        p = (p | (p << 4)) & 0x0f0f0f0fu;
+        p = (p | (p << 2)) & 0x33333333u;  // nibble per field
+        // e fields in the lower half, o fields in the upper: byte q = e_q | o_q << 4
+        const uint32_t lo16 = p & 0xffffu, hi16 = p >> 16;
+        uint32_t be = (lo16 | (lo16 << 8)) & 0x00ff00ffu, bo = (hi16 | (hi16 << 8)) & 0x00ff00ffu;
+        be = (be | (be << 4)) & 0x0f0f0f0fu;
+        bo = (bo | (bo << 4)) & 0x0f0f0f0fu;
+        bytes[h] = (be | (bo << 4)) << (2 * tpar);
+      }
     }
     if (tpar == 1) {
       xch[grp][lane][0] = bytes[0];
       xch[grp][lane][1] = bytes[1];
     }
     __syncthreads();
-    if (tpar == 0 && colok) {
+    if (tpar == 0 && colok && obase < nout) {
       bytes[0] |= xch[grp][lane][0];
       bytes[1] |= xch[grp][lane][1];
-      const int cx = x >> 1, cy = third >> 1;
+      uint8_t* dst = out8 + idx3(x >> 1, third >> 1, obase / 2, rx, ry);
 #pragma unroll
-      for (int q = 0; q < kDpxPer / 2; q++) {
-        const int cz = obase / 2 + q;
-        if (2 * cz < N) out8[idx3(cx, cy, cz, rx, ry)] = (uint8_t)((bytes[q >> 2] >> (8 * (q & 3))) & 0xffu);
-      }
+      for (int q = 0; q < kDpxPer / 2; q++)
+        dst[(int64_t)rx * ry * q] = (uint8_t)((bytes[q >> 2] >> (8 * (q & 3))) & 0xffu);
     }
   }
 }
@@ -1217,10 +1240,9 @@ __global__ void __launch_bounds__(256, 4) k_pass_dpx(const TIn* __restrict__ in,
                                                   uint8_t* __restrict__ out8, int nx, int ny, int nz, int axis,
                                                   int sub, int halo, uint32_t cap, RField R,
                                                   int uniform_r, int rx, int ry, const uint8_t* __restrict__ rmap,
-                                                  int rext, NeedMap need, const __grid_constant__ CUtensorMap tmap,
-                                                  int use_tma) {
+                                                  int rext, const __grid_constant__ NeedMap need) {
   dpx_tile<G, TIn, FIN>(in, out16, out8, nx, ny, nz, axis, sub, halo, cap, R, uniform_r, rx, ry, rmap, rext, need,
-                        &tmap, use_tma, (int)blockIdx.x, (int)blockIdx.y + need.out0, (int)blockIdx.z + need.third0);
+                        (int)blockIdx.x, (int)blockIdx.y + need.out0, (int)blockIdx.z + need.third0);
 }
 
 template <int G, typename TIn, int FIN>
@@ -1236,24 +1258,9 @@ static void launch_dpx(const TIn* in, uint16_t* out16, uint8_t* out8, int nx, in
   const int nout = sub ? na / 2 : na;
   dim3 g((nx + kDpxCols - 1) / kDpxCols, need.out_n > 0 ? need.out_n : (nout + kDpxOut - 1) / kDpxOut,
          need.third_n > 0 ? need.third_n : (n3 + 1) / 2);
-  // Full-resolution u16 tiles go through TMA (one box of the whole span per
-  // third-axis slice) when the field's rows are whole 64-column boxes.
-  // Measured at 1024^3: dilation z 2.71 -> 2.64 ms, centre erosion y
-  // 1.27 -> 1.24 ms; the half-resolution lattice passes (sub) were a third
-  // slower with TMA (0.63 -> 0.84, 0.31 -> 0.42 ms; 16-row boxes: slower
-  // everywhere) and keep their per-thread loads.
-  CUtensorMap tmap;
-  memset(&tmap, 0, sizeof(tmap));
-  int use_tma = 0;
-  const int span = (sub ? 2 * kDpxOut - 1 : kDpxOut) + 2 * halo;
-  if (sizeof(TIn) == 2 && sub == 0 && nx % kDpxCols == 0 && span <= 256 &&
-      (reinterpret_cast<uintptr_t>(in) & 15) == 0)
-    use_tma = encode_tensor_map_3d(&tmap, in, 2, nx, ny, nz, kDpxCols, axis == 1 ? span : 1, axis == 1 ? 1 : span)
-                  ? 1
-                  : 0;
   GM_LAUNCH(kc, name, st,
             k_pass_dpx<G, TIn, FIN><<<g, 256, smem, st>>>(in, out16, out8, nx, ny, nz, axis, sub, halo, cap, R,
-                                                          uniform_r, rx, ry, rmap, rext, need, tmap, use_tma));
+                                                          uniform_r, rx, ry, rmap, rext, need));
 }
 
 // ---- grouped min-plus passes (many grids, one persistent launch) ----
@@ -1348,8 +1355,7 @@ __global__ void __launch_bounds__(256, 4) k_pass_dpx_group(const DpxJob* __restr
     const int t = item - b.first;
     const int bx = t % b.gx, by = (t / b.gx) % b.gy, bz = t / (b.gx * b.gy);
     dpx_tile<G, TIn, FIN>(static_cast<const TIn*>(b.in), b.out16, b.out8, b.nx, b.ny, b.nz, b.axis, b.sub, b.halo,
-                          b.cap, b.R, b.uniform_r, b.rx, b.ry, b.rmap, b.rext, b.need, nullptr, 0,
-                          bx, by + b.need.out0, bz + b.need.third0);
+                          b.cap, b.R, b.uniform_r, b.rx, b.ry, b.rmap, b.rext, b.need, bx, by + b.need.out0, bz + b.need.third0);
     __syncthreads();  // every thread is done with this tile (its shared memory, job_s, item_s)
     if (threadIdx.x == 0) item_s = next;
     __syncthreads();
@@ -1518,39 +1524,6 @@ static bool dpx_step(const CloseArgs& a, int& at, const TIn* in, uint16_t* out16
                                                         uniform_r, rx, ry, rmap, rext, need);
   at++;
   return ok;
-}
-
-// The driver's tensor-map encoder, looked up once per process (before any
-// stream capture: gm_ctx_create calls tma_init).
-static PFN_cuTensorMapEncodeTiled_v12000 tma_encoder() {
-  static std::once_flag once;
-  static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
-  std::call_once(once, [] {
-    void* fn = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &q) ==
-            cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
-    cudaGetLastError();
-  });
-  return encode;
-}
-
-void tma_init() { tma_encoder(); }
-
-bool encode_tensor_map_3d(CUtensorMap* map, const void* base, int elem_bytes, int nx, int ny, int nz, int bx, int by,
-                          int bz) {
-  const PFN_cuTensorMapEncodeTiled_v12000 encode = tma_encoder();
-  if (encode == nullptr || (elem_bytes != 1 && elem_bytes != 2)) return false;
-  const cuuint64_t dims[3] = {(cuuint64_t)nx, (cuuint64_t)ny, (cuuint64_t)nz};
-  const cuuint64_t strides[2] = {(cuuint64_t)nx * elem_bytes, (cuuint64_t)nx * ny * elem_bytes};
-  const cuuint32_t box[3] = {(cuuint32_t)bx, (cuuint32_t)by, (cuuint32_t)bz};
-  const cuuint32_t estr[3] = {1, 1, 1};
-  return encode(map, elem_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_UINT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 3,
-                const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 cudaError_t kernel_error_flags(unsigned int* flags, bool clear) {
