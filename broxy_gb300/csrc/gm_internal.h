@@ -260,18 +260,16 @@ struct MeshBuffers {
   void release();
   float* V = nullptr;       // 3 * v_cap
   float* N = nullptr;       // 3 * v_cap
-  float* N2 = nullptr;      // unused (kept for ABI-stable layout of the struct)
   float4* N4a = nullptr;    // v_cap, bilateral ping-pong (16-byte normals)
   float4* N4b = nullptr;    // v_cap
-  uint2* ent = nullptr;     // 6 * t_cap: filter records as built, vertex v's from 2 rowptr[v] (a
-                            // neighbour and its position term |pa-pb|^2, float bits; the sign bit
-                            // set when two incident triangles share the neighbour)
-  uint2* rec = nullptr;     // 6 * t_cap: the same records packed, vertex v's at [roff[v], roff[v+1])
-  uint32_t* roff = nullptr; // v_cap + 1
+  uint2* rec = nullptr;     // 6 * t_cap: filter records (a neighbour and its position term |pa-pb|^2,
+                            // float bits; the sign bit set when two incident triangles share the
+                            // neighbour), packed in chunks of 256 vertices
+  uint32_t* roff = nullptr; // v_cap + v_cap / 256 + 4: their offsets, 257 a chunk after vertex 0's two
   uint32_t* T = nullptr;    // 3 * t_cap
-  uint32_t* adj = nullptr;  // 3 * t_cap (vertex -> corner list)
-  uint32_t* rowptr = nullptr;  // v_cap + 1
-  uint32_t* cursor = nullptr;  // v_cap
+  uint32_t* row0 = nullptr; // 3 * t_cap: corners of vertex 0 where they are many
+  uint32_t* adj = nullptr;  // 20 * v_cap: corner rows (8 slots a vertex, then 12 more each)
+  uint32_t* cursor = nullptr;  // v_cap corner counts, then the mesh's counters
   int64_t v_cap = 0, t_cap = 0;
   // per-cell / per-brick scratch
   uint32_t* cell_voff = nullptr;  // res^3

@@ -687,159 +687,40 @@ __global__ void k_mc_fix91(const uint32_t* __restrict__ fix, int fix_cap, uint32
 
 // ------------------------------------------------------------------ normals
 
-// Vertex -> corner lists.  Corners of a vertex are listed in corner order
-// (the reference's per-vertex accumulation order).  Vertex 0 is special: the
-// reference's triangles take index 0 for an edge whose owning cube is not
-// tagged (cubes of border cells), so on grids whose surface reaches the
-// border vertex 0 collects an unbounded number of corners.  Its row is
-// built by an order-preserving compaction over all corners (linear), the
-// other rows (at most 20 corners each) by atomics and an in-row sort.
-__global__ void k_adj_count(const uint32_t* __restrict__ T, int64_t nt, uint32_t* __restrict__ cnt) {
+// Vertex -> corner lists.  A vertex sits on an edge shared by four cubes of
+// at most five triangles, so it has at most kAdjMax corners and its list is
+// a row of fixed size: one pass of atomics fills it, in any order, and
+// k_adj_finish sorts it (no counting pass, no scan).  The first kAdjRow
+// slots (32 bytes, enough for nearly every vertex) and the others are
+// separate arrays.  Vertex 0 is special: the reference's triangles take
+// index 0 for an edge whose owning cube is not tagged (cubes of border
+// cells), so on grids whose surface reaches the border vertex 0 collects an
+// unbounded number of corners; past kAdjMax they are collected apart.
+constexpr int kAdjMax = 20;
+constexpr int kAdjRow = 8;
+
+// counters after the vertices' in `cursor`: corners of vertex 0 collected,
+// records placed
+enum { kCntRow0 = 0, kCntRecords = 1, kCntWords = 4 };
+
+__global__ void k_adj_slots(const uint32_t* __restrict__ T, int64_t nt, uint32_t* __restrict__ cursor,
+                            uint32_t* __restrict__ adj, uint32_t* __restrict__ adj_more) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < 3 * nt; i += (int64_t)gridDim.x * blockDim.x) {
     const uint32_t v = T[i];
-    if (v != 0u) atomicAdd(cnt + v, 1u);
-  }
-}
-
-constexpr int kRow0Chunk = 2048;  // corners per block (256 threads x 8)
-
-// corners of vertex 0 per chunk of kRow0Chunk corners
-__global__ void __launch_bounds__(256) k_row0_count(const uint32_t* __restrict__ T, int64_t n,
-                                                     uint32_t* __restrict__ counts) {
-  __shared__ uint32_t ws[8];
-  const int64_t base = (int64_t)blockIdx.x * kRow0Chunk;
-  uint32_t c = 0;
-  for (int i = threadIdx.x; i < kRow0Chunk; i += 256)
-    if (base + i < n) c += T[base + i] == 0u;
-  for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = c;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    uint32_t t = 0;
-    for (int w = 0; w < 8; w++) t += ws[w];
-    counts[blockIdx.x] = t;
-  }
-}
-
-// the count of vertex 0 (total of the scanned chunk counts) into cnt[0]
-__global__ void k_row0_total(const uint32_t* __restrict__ offs, int nchunks, uint32_t* __restrict__ cnt) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) cnt[0] = offs[nchunks];
-}
-
-// row 0 in corner order: chunk offset + rank inside the chunk
-__global__ void __launch_bounds__(256) k_row0_fill(const uint32_t* __restrict__ T, int64_t n,
-                                                    const uint32_t* __restrict__ offs,
-                                                    const uint32_t* __restrict__ rowptr, uint32_t* __restrict__ adj) {
-  __shared__ uint32_t wtot[8];
-  const int64_t base = (int64_t)blockIdx.x * kRow0Chunk + (int64_t)threadIdx.x * 8;
-  uint32_t f = 0, s = 0;
-#pragma unroll
-  for (int j = 0; j < 8; j++) {
-    const bool z = base + j < n && T[base + j] == 0u;
-    f |= (z ? 1u : 0u) << j;
-    s += z ? 1u : 0u;
-  }
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  uint32_t x = s;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t t = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += t;
-  }
-  if (lane == 31) wtot[wid] = x;
-  __syncthreads();
-  uint32_t pos = rowptr[0] + offs[blockIdx.x] + x - s;
-  for (int w = 0; w < wid; w++) pos += wtot[w];
-#pragma unroll
-  for (int j = 0; j < 8; j++)
-    if ((f >> j) & 1u) adj[pos++] = (uint32_t)(base + j);
-}
-
-// Exclusive scan of n u32 into out[0..n] in three kernels: per-block sums of
-// 2048-element chunks, a scan of the block sums, then per-chunk scans.
-constexpr int kScanChunk = 2048;
-
-__global__ void __launch_bounds__(256) k_scan_sums(const uint32_t* __restrict__ in, int64_t n,
-                                                    uint32_t* __restrict__ sums) {
-  __shared__ uint32_t ws[8];
-  const int64_t base = (int64_t)blockIdx.x * kScanChunk;
-  uint32_t s = 0;
-  for (int i = threadIdx.x; i < kScanChunk; i += 256)
-    if (base + i < n) s += in[base + i];
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    uint32_t t = 0;
-    for (int w = 0; w < 8; w++) t += ws[w];
-    sums[blockIdx.x] = t;
-  }
-}
-
-__global__ void __launch_bounds__(1024) k_scan_small(uint32_t* __restrict__ v, int n) {
-  __shared__ uint32_t part[1024];
-  const int t = threadIdx.x;
-  const int per = (n + 1023) / 1024;
-  const int b0 = t * per, b1 = min(n, b0 + per);
-  uint32_t s = 0;
-  for (int b = b0; b < b1; b++) s += v[b];
-  part[t] = s;
-  __syncthreads();
-  for (int o = 1; o < 1024; o <<= 1) {
-    const uint32_t x = t >= o ? part[t - o] : 0;
-    __syncthreads();
-    part[t] += x;
-    __syncthreads();
-  }
-  uint32_t run = part[t] - s;
-  for (int b = b0; b < b1; b++) {
-    const uint32_t x = v[b];
-    v[b] = run;
-    run += x;
-  }
-  if (t == 1023) v[n] = part[1023];
-}
-
-__global__ void __launch_bounds__(256) k_scan_apply(const uint32_t* __restrict__ in, int64_t n,
-                                                     const uint32_t* __restrict__ sums, uint32_t* __restrict__ out) {
-  __shared__ uint32_t wtot[8];
-  const int64_t base = (int64_t)blockIdx.x * kScanChunk + (int64_t)threadIdx.x * 8;
-  uint32_t v[8], s = 0;
-#pragma unroll
-  for (int j = 0; j < 8; j++) {
-    v[j] = base + j < n ? in[base + j] : 0u;
-    s += v[j];
-  }
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  uint32_t x = s;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t t = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += t;
-  }
-  if (lane == 31) wtot[wid] = x;
-  __syncthreads();
-  uint32_t wpre = 0;
-  for (int w = 0; w < wid; w++) wpre += wtot[w];
-  uint32_t run = sums[blockIdx.x] + wpre + x - s;
-#pragma unroll
-  for (int j = 0; j < 8; j++) {
-    if (base + j < n) out[base + j] = run;
-    run += v[j];
-  }
-  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 255) out[n] = sums[gridDim.x];
-}
-
-__global__ void k_adj_fill(const uint32_t* __restrict__ T, int64_t nt, const uint32_t* __restrict__ rowptr,
-                           uint32_t* __restrict__ cursor, uint32_t* __restrict__ adj) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < 3 * nt; i += (int64_t)gridDim.x * blockDim.x) {
-    const uint32_t v = T[i];
-    if (v == 0u) continue;  // row 0: k_row0_fill
     const uint32_t slot = atomicAdd(cursor + v, 1u);
-    adj[rowptr[v] + slot] = (uint32_t)i;  // corner id = 3 t + role
+    if (slot < kAdjRow) adj[(size_t)kAdjRow * v + slot] = (uint32_t)i;  // corner id = 3 t + role
+    else if (slot < kAdjMax) adj_more[(size_t)(kAdjMax - kAdjRow) * v + slot - kAdjRow] = (uint32_t)i;
   }
 }
 
+// The corners of a vertex 0 that has more than kAdjMax of them (else nothing
+// to do), in any order.
+__global__ void k_row0_collect(const uint32_t* __restrict__ T, int64_t nt, const uint32_t* __restrict__ cursor,
+                               uint32_t* __restrict__ counters, uint32_t* __restrict__ row0) {
+  if (cursor[0] <= kAdjMax) return;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < 3 * nt; i += (int64_t)gridDim.x * blockDim.x)
+    if (T[i] == 0u) row0[atomicAdd(counters + kCntRow0, 1u)] = (uint32_t)i;
+}
 
 __device__ __forceinline__ float3 ld3(const float* p, uint32_t i) {
   return make_float3(p[3 * (size_t)i], p[3 * (size_t)i + 1], p[3 * (size_t)i + 2]);
@@ -862,17 +743,7 @@ __device__ __forceinline__ float dist2n(float4 a, float4 b) {
   return __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
 }
 
-// The per-vertex steps after the incident-triangle lists are filled, in
-// one kernel: the list sorted into triangle order (in registers, a bitonic
-// network over 8 or 16 slots; vertex 0's row is already in order, longer
-// lists are sorted in place); the area-weighted normal (ComputeMeshNormals,
-// GMorpho.cu:6498-6524) summed in that order and normalised
-// (GMorpho.cu:6526-6537); and, when the normals are filtered, each corner's
-// filter record: the other two vertices b, c in the reference's order and
-// the iteration-invariant position terms |pa - pb|^2 / sigma_p^2
-// (GMorpho.cu:6561-6569) — sigma_p is 1 (GMorpho.cu:6959-6969), so the term
-// is the squared distance itself (an IEEE division by 1 is exact).  Every
-// incident triangle's vertices and positions are loaded once for both.
+// Compare-exchange networks over M values in registers.
 template <int M>
 __device__ __forceinline__ void bitonic_sort(uint32_t (&k)[M]) {
 #pragma unroll
@@ -891,158 +762,252 @@ __device__ __forceinline__ void bitonic_sort(uint32_t (&k)[M]) {
       }
 }
 
-// one incident corner: its triangle's normal term, and its filter record
+// one incident corner: its triangle's other vertices, the one after it and
+// the one before it in the triangle's orientation, and its normal term
+// (ComputeMeshNormals, GMorpho.cu:6498-6524)
 __device__ __forceinline__ void adj_corner(const float* __restrict__ V, const uint32_t* __restrict__ T,
-                                           uint32_t corner, const float3& pa, float3& acc, uint64_t* pair) {
+                                           uint32_t corner, float3& n, uint32_t& next, uint32_t& prev) {
   const uint32_t t = corner / 3, role = corner - 3 * t;
   const uint32_t i0 = T[3 * (size_t)t], i1 = T[3 * (size_t)t + 1], i2 = T[3 * (size_t)t + 2];
   const float3 p0 = ld3(V, i0), p1 = ld3(V, i1), p2 = ld3(V, i2);
   const float3 a = make_float3(__fsub_rn(p1.x, p0.x), __fsub_rn(p1.y, p0.y), __fsub_rn(p1.z, p0.z));
   const float3 b = make_float3(__fsub_rn(p2.x, p0.x), __fsub_rn(p2.y, p0.y), __fsub_rn(p2.z, p0.z));
-  const float nx = __fsub_rn(__fmul_rn(a.y, b.z), __fmul_rn(a.z, b.y));
-  const float ny = __fsub_rn(__fmul_rn(a.z, b.x), __fmul_rn(a.x, b.z));
-  const float nz = __fsub_rn(__fmul_rn(a.x, b.y), __fmul_rn(a.y, b.x));
-  acc = make_float3(__fadd_rn(acc.x, nx), __fadd_rn(acc.y, ny), __fadd_rn(acc.z, nz));
-  if (pair) {
-    // the other two vertices (reference order (1, 2), (0, 2), (0, 1)) as
-    // (vertex << 32 | position term bits)
-    const uint32_t ib = role == 0 ? i1 : i0, ic = role == 2 ? i1 : i2;
-    const float3 pb = role == 0 ? p1 : p0, pc = role == 2 ? p1 : p2;
-    pair[0] = ((uint64_t)ib << 32) | __float_as_uint(dist2(pa, pb));
-    pair[1] = ((uint64_t)ic << 32) | __float_as_uint(dist2(pa, pc));
-  }
+  n.x = __fsub_rn(__fmul_rn(a.y, b.z), __fmul_rn(a.z, b.y));
+  n.y = __fsub_rn(__fmul_rn(a.z, b.x), __fmul_rn(a.x, b.z));
+  n.z = __fsub_rn(__fmul_rn(a.x, b.y), __fmul_rn(a.y, b.x));
+  next = role == 0 ? i1 : (role == 1 ? i2 : i0);
+  prev = role == 0 ? i2 : (role == 1 ? i0 : i1);
 }
 
-template <int M>
-__device__ __forceinline__ void bitonic_sort64(uint64_t (&k)[M]) {
-#pragma unroll
-  for (int s = 2; s <= M; s <<= 1)
-#pragma unroll
-    for (int j = s >> 1; j > 0; j >>= 1)
-#pragma unroll
-      for (int i = 0; i < M; i++) {
-        const int l = i ^ j;
-        if (l > i) {
-          const uint64_t a = k[i], b = k[l];
-          const bool up = (i & s) == 0;
-          k[i] = up ? (a < b ? a : b) : (a < b ? b : a);
-          k[l] = up ? (a < b ? b : a) : (a < b ? a : b);
-        }
-      }
+__device__ __forceinline__ float3 add3(float3 a, float3 b) {
+  return make_float3(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y), __fadd_rn(a.z, b.z));
 }
 
-// The filter records of a vertex from its neighbour pairs sorted by
-// (vertex, term): one record per neighbour, or per two occurrences of it
-// (an edge shared by two incident triangles), the sign bit marking a
-// double.  Returns the number of records written.
-__device__ __forceinline__ uint32_t put_records(const uint64_t* kv, int m, uint2* rec) {
-  uint32_t w = 0;
+// Filter records of a vertex: (neighbour, position term bits |pa - pb|^2),
+// one per neighbour or per two occurrences of it among the incident
+// triangles (an edge shared by two of them), the sign bit marking a double;
+// in (neighbour, term) order.  sigma_p is 1 (GMorpho.cu:6959-6969), so the
+// term of GMorpho.cu:6561-6569 is the squared distance itself.
+//
+// The records of kRecChunk consecutive vertices are packed, the chunks in
+// any order (each takes its place from a counter: no scan over the mesh);
+// a chunk has its own row of offsets, one more than its vertices, after
+// vertex 0's own start and end (its records may lie apart).  (The
+// iterations are bound by the records' bytes and the gathers' latency: rows
+// of eight slots a vertex, or slots of 32 vertices interleaved, were 18%
+// slower.)
+constexpr int kRecChunk = 256;
+__device__ __forceinline__ uint32_t roff_at(uint32_t v) { return v == 0u ? 0u : v + v / kRecChunk + 2u; }
+
+// pairs (neighbour << 32 | term bits) sorted; merged in place into records
+// (they never overtake the pairs still to be read); returns how many
+__device__ uint32_t merge_pairs(uint64_t* kv, uint32_t m) {
+  uint32_t w = 0, prev = 0;
   int run = 0;
-  for (int i = 0; i < m; i++) {
-    if (kv[i] == ~0ull) break;
-    run = (i > 0 && (kv[i] >> 32) == (kv[i - 1] >> 32)) ? run + 1 : 0;
+  for (uint32_t i = 0; i < m; i++) {
+    const uint64_t x = kv[i];
+    const uint32_t id = (uint32_t)(x >> 32);
+    run = (i > 0 && id == prev) ? run + 1 : 0;
+    prev = id;
     if (run & 1) continue;
-    const bool dbl = i + 1 < m && kv[i + 1] != ~0ull && (kv[i + 1] >> 32) == (kv[i] >> 32);
-    rec[w++] = make_uint2((uint32_t)(kv[i] >> 32), (uint32_t)kv[i] | (dbl ? 0x80000000u : 0u));
+    const bool dbl = i + 1 < m && (uint32_t)(kv[i + 1] >> 32) == id;
+    kv[w++] = ((uint64_t)id << 32) | (uint32_t)x | (dbl ? 0x80000000u : 0u);
   }
   return w;
 }
+__device__ __forceinline__ uint2 as_record(uint64_t kv) { return make_uint2((uint32_t)(kv >> 32), (uint32_t)kv); }
 
-__global__ void __launch_bounds__(256, 4) k_adj_finish(const float* __restrict__ V, const uint32_t* __restrict__ T,
-                             const uint32_t* __restrict__ rowptr, uint32_t* __restrict__ adj, int64_t nv,
+// A vertex in general: more than kAdjRow corners, or a surface around it
+// that is not a closed fan.  Returns its normal sum; its records to kv.
+__device__ __noinline__ float3 finish_general(const float* __restrict__ V, const uint32_t* __restrict__ T, int64_t v,
+                                              uint32_t n, const uint32_t* __restrict__ adj,
+                                              const uint32_t* __restrict__ adj_more, float3 pa, uint64_t* kv,
+                                              uint32_t* records) {
+  uint32_t key[kAdjMax];
+  for (uint32_t i = 0; i < n; i++) {
+    const uint32_t c = i < kAdjRow ? adj[(size_t)kAdjRow * v + i]
+                                   : adj_more[(size_t)(kAdjMax - kAdjRow) * v + i - kAdjRow];
+    uint32_t j = i;
+    while (j > 0 && key[j - 1] > c) { key[j] = key[j - 1]; j--; }
+    key[j] = c;
+  }
+  float3 acc = make_float3(0.f, 0.f, 0.f);
+  uint32_t m = 0;
+  for (uint32_t i = 0; i < n; i++) {
+    float3 nn;
+    uint32_t id[2];
+    adj_corner(V, T, key[i], nn, id[0], id[1]);
+    acc = add3(acc, nn);
+    for (int h = 0; h < 2; h++) {
+      const uint64_t x = ((uint64_t)id[h] << 32) | __float_as_uint(dist2(pa, ld3(V, id[h])));
+      uint32_t j = m++;
+      while (j > 0 && kv[j - 1] > x) { kv[j] = kv[j - 1]; j--; }
+      kv[j] = x;
+    }
+  }
+  *records = merge_pairs(kv, m);
+  return acc;
+}
+
+// The per-vertex steps after the corner rows are filled, in one kernel: the
+// row sorted into triangle order; the area-weighted normal summed in that
+// order and normalised (GMorpho.cu:6498-6537); and, when the normals are
+// filtered (rec), the filter records.
+//
+// Around a vertex whose triangles form closed fans, every neighbour follows
+// it in one incident triangle and precedes it in another: the sorted lists
+// of both are equal, and each entry is a neighbour shared by two triangles.
+// Two networks over eight 32-bit values and a comparison thus replace the
+// sort of sixteen 64-bit pairs, and the records go straight to their packed
+// place: with the corner rows' single pass, 4.4M vertices' lists and records
+// went from 1.27 ms (count, scan, fill, finish, scan, pack) to 0.6.
+__global__ void __launch_bounds__(kRecChunk, 4) k_adj_finish(const float* __restrict__ V, const uint32_t* __restrict__ T,
+                             const uint32_t* __restrict__ cursor, const uint32_t* __restrict__ adj,
+                             const uint32_t* __restrict__ adj_more, int64_t nv,
                              int zero_isolated, float4* __restrict__ N4, float* __restrict__ N3,
-                             uint2* __restrict__ ent, uint32_t* __restrict__ ncnt) {
-  for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < nv; v += (int64_t)gridDim.x * blockDim.x) {
-    const uint32_t b = rowptr[v], e = rowptr[v + 1], n = e - b;
-    if (zero_isolated && n == 0) {
-      N4[v] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (N3) { N3[3 * v] = 0.f; N3[3 * v + 1] = 0.f; N3[3 * v + 2] = 0.f; }
-      if (ent) ncnt[v] = 0;
-      continue;
+                             uint2* __restrict__ rec, uint32_t* __restrict__ roff, uint32_t* __restrict__ counters) {
+  __shared__ uint32_t base_s;
+  const int64_t v = blockIdx.x * (int64_t)kRecChunk + threadIdx.x;
+  const uint32_t n = v < nv ? cursor[v] : 0u;
+  const bool isolated = n == 0 && (zero_isolated || v >= nv);
+  const bool here = !isolated && n <= kAdjMax;  // (more: vertex 0, k_row0_finish)
+  float3 acc = make_float3(0.f, 0.f, 0.f);
+  uint32_t p[8], t[8], records = 0;
+  uint64_t kv[2 * kAdjMax];
+  bool fan = here && n <= kAdjRow;
+  if (fan) {
+    uint32_t key[8], q[8];
+    const uint4* row = reinterpret_cast<const uint4*>(adj + (size_t)kAdjRow * v);
+    const uint4 r0 = row[0], r1 = row[1];
+    key[0] = r0.x, key[1] = r0.y, key[2] = r0.z, key[3] = r0.w;
+    key[4] = r1.x, key[5] = r1.y, key[6] = r1.z, key[7] = r1.w;
+#pragma unroll
+    for (int k = 0; k < 8; k++) key[k] = (uint32_t)k < n ? key[k] : 0xffffffffu;
+    bitonic_sort<8>(key);
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      p[k] = q[k] = 0xffffffffu;
+      if ((uint32_t)k < n) {
+        float3 nn;
+        adj_corner(V, T, key[k], nn, p[k], q[k]);
+        acc = add3(acc, nn);
+      }
     }
-    const float3 pa = ld3(V, (uint32_t)v);
-    float3 acc = make_float3(0.f, 0.f, 0.f);
-    if (v != 0 && n <= 8) {
-      uint32_t key[8];
-      uint64_t kv[16];
+    if (rec) {
+      bitonic_sort<8>(p);
+      bitonic_sort<8>(q);
 #pragma unroll
-      for (int k = 0; k < 8; k++) key[k] = (uint32_t)k < n ? adj[b + k] : 0xffffffffu;
-      bitonic_sort<8>(key);
+      for (int k = 0; k < 8; k++) fan = fan && p[k] == q[k];
+      if (fan) {
+        const float3 pa = ld3(V, (uint32_t)v);
+        records = n;
 #pragma unroll
-      for (int k = 0; k < 8; k++) {
-        kv[2 * k] = kv[2 * k + 1] = ~0ull;
-        if ((uint32_t)k < n) {
-          adj[b + k] = key[k];
-          adj_corner(V, T, key[k], pa, acc, ent ? kv + 2 * k : nullptr);
-        }
+        for (int k = 0; k < 8; k++)
+          if ((uint32_t)k < n) t[k] = __float_as_uint(dist2(pa, ld3(V, p[k]))) | 0x80000000u;
       }
-      if (ent) {
-        bitonic_sort64<16>(kv);
-        ncnt[v] = put_records(kv, 16, ent + 2 * (size_t)b);
-      }
+    }
+  }
+  if (here && !fan) acc = finish_general(V, T, v, n, adj, adj_more, ld3(V, (uint32_t)v), kv, &records);
+  if (rec) {
+    uint32_t total;
+    const uint32_t pre = block_scan1(records, total);
+    if (threadIdx.x == 0) base_s = atomicAdd(counters + kCntRecords, total);
+    __syncthreads();
+    const uint32_t at = base_s + pre;
+    if (v < nv && n <= kAdjMax) {
+      roff[roff_at((uint32_t)v)] = at;
+      if (v == 0 || threadIdx.x == kRecChunk - 1 || v == nv - 1) roff[roff_at((uint32_t)v) + 1] = at + records;
+    }
+    if (fan) {
+#pragma unroll
+      for (int k = 0; k < 8; k++)
+        if ((uint32_t)k < records) rec[at + k] = make_uint2(p[k], t[k]);
     } else {
-      // rare (more than 8 incident triangles): sorted in memory
-      if (v != 0)
-        for (uint32_t i = b + 1; i < e; i++) {  // in place (vertex 0's row is already in order)
-          const uint32_t key = adj[i];
-          uint32_t j = i;
-          while (j > b && adj[j - 1] > key) { adj[j] = adj[j - 1]; j--; }
-          adj[j] = key;
-        }
-      // the pairs in the record slots, sorted there, then merged in place
-      uint64_t* kv = ent ? reinterpret_cast<uint64_t*>(ent + 2 * (size_t)b) : nullptr;
-      for (uint32_t i = b; i < e; i++) adj_corner(V, T, adj[i], pa, acc, kv ? kv + 2 * (i - b) : nullptr);
-      if (kv) {
-        const uint32_t m = 2 * n;
-        for (uint32_t i = 1; i < m; i++) {
-          const uint64_t x = kv[i];
-          uint32_t j = i;
-          while (j > 0 && kv[j - 1] > x) { kv[j] = kv[j - 1]; j--; }
-          kv[j] = x;
-        }
-        // merged records never overtake the pairs still to be read
-        uint32_t w = 0;
-        int run = 0;
-        uint32_t prev = 0;
-        for (uint32_t i = 0; i < m; i++) {
-          const uint64_t x = kv[i];
-          const uint32_t id = (uint32_t)(x >> 32);
-          run = (i > 0 && id == prev) ? run + 1 : 0;
-          prev = id;
-          if (run & 1) continue;
-          const bool dbl = i + 1 < m && (uint32_t)(kv[i + 1] >> 32) == id;
-          ent[2 * (size_t)b + w++] = make_uint2(id, (uint32_t)x | (dbl ? 0x80000000u : 0u));
-        }
-        ncnt[v] = w;
-      }
+      for (uint32_t i = 0; i < records; i++) rec[at + i] = as_record(kv[i]);
     }
-    const float3 nn = normalize3(acc);
-    N4[v] = make_float4(nn.x, nn.y, nn.z, 0.f);
-    if (N3) { N3[3 * v] = nn.x; N3[3 * v + 1] = nn.y; N3[3 * v + 2] = nn.z; }
+  }
+  if (v >= nv || !(here || isolated)) return;
+  float3 nn = make_float3(0.f, 0.f, 0.f);
+  if (here) nn = normalize3(acc);
+  N4[v] = make_float4(nn.x, nn.y, nn.z, 0.f);
+  if (N3) { N3[3 * v] = nn.x; N3[3 * v + 1] = nn.y; N3[3 * v + 2] = nn.z; }
+}
+
+// Ascending sort of n values in global memory by one block (a bitonic
+// network whose exchanges all put the smaller value first, so that the
+// places past n need no padding).
+template <typename K>
+__device__ void block_sort(K* k, uint32_t n) {
+  for (uint32_t s = 2; s / 2 < n; s <<= 1) {
+    for (uint32_t j = s >> 1; j > 0; j >>= 1) {
+      for (uint32_t t = threadIdx.x; t < n; t += blockDim.x) {
+        // the first step of a merge mirrors the second half
+        const uint32_t l = j == s >> 1 ? (t & ~(s - 1)) + (s - 1 - (t & (s - 1))) : t ^ j;
+        if (l > t && l < n) {
+          const K a = k[t], b = k[l];
+          if (b < a) k[t] = b, k[l] = a;
+        }
+      }
+      __syncthreads();
+    }
   }
 }
 
-// Packs each vertex's records (built from 2 rowptr[v], roff from the scan
-// of their counts) so that the iterations read them contiguously.
-__global__ void k_rec_pack(const uint2* __restrict__ ent, const uint32_t* __restrict__ rowptr,
-                           const uint32_t* __restrict__ roff, int64_t nv, uint2* __restrict__ rec) {
-  for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < nv; v += (int64_t)gridDim.x * blockDim.x) {
-    const uint2* src = ent + 2 * (size_t)rowptr[v];
-    const uint32_t r0 = roff[v], n = roff[v + 1] - r0;
-    for (uint32_t i = 0; i < n; i++) rec[r0 + i] = src[i];
+// Vertex 0 with more than kAdjMax corners (else nothing to do): the steps of
+// k_adj_finish by one block, the terms in parallel and their sum in corner
+// order by one thread.  Its pairs and then its records lie at the end of the
+// records' buffer (the other vertices' fill it from the front; together they
+// are at most two a corner).
+__global__ void __launch_bounds__(1024) k_row0_finish(const float* __restrict__ V, const uint32_t* __restrict__ T,
+                                                      const uint32_t* __restrict__ cursor, uint32_t* __restrict__ row0,
+                                                      int64_t nt, float4* __restrict__ N4, float* __restrict__ N3,
+                                                      uint2* __restrict__ rec, uint32_t* __restrict__ roff) {
+  const uint32_t n = cursor[0];
+  if (n <= kAdjMax) return;
+  __shared__ float3 term[1024];
+  block_sort(row0, n);
+  const uint32_t start = (uint32_t)(6 * nt - 2 * (int64_t)n);
+  uint64_t* kv = reinterpret_cast<uint64_t*>(rec + start);  // (8 bytes a record, 8 bytes a pair)
+  const float3 pa = ld3(V, 0u);
+  float3 acc = make_float3(0.f, 0.f, 0.f);
+  for (uint32_t c0 = 0; c0 < n; c0 += blockDim.x) {
+    const uint32_t c = c0 + threadIdx.x;
+    if (c < n) {
+      uint32_t id[2];
+      adj_corner(V, T, row0[c], term[threadIdx.x], id[0], id[1]);
+      if (rec)
+        for (int h = 0; h < 2; h++)
+          kv[2 * (size_t)c + h] = ((uint64_t)id[h] << 32) | __float_as_uint(dist2(pa, ld3(V, id[h])));
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+      for (uint32_t i = 0; i < blockDim.x && c0 + i < n; i++) acc = add3(acc, term[i]);
+    __syncthreads();
   }
+  if (rec) block_sort(kv, 2 * n);
+  if (threadIdx.x != 0) return;
+  if (rec) {
+    const uint32_t w = merge_pairs(kv, 2 * n);
+    for (uint32_t i = 0; i < w; i++) kv[i] = (kv[i] << 32) | (kv[i] >> 32);  // a record's word order
+    roff[0] = start;
+    roff[1] = start + w;
+  }
+  const float3 nn = normalize3(acc);
+  N4[0] = make_float4(nn.x, nn.y, nn.z, 0.f);
+  if (N3) { N3[0] = nn.x; N3[1] = nn.y; N3[2] = nn.z; }
 }
 
 // One bilateral normal iteration (BilateralMeshFiltering{,Normalize},
 // GMorpho.cu:6539-6620): each incident triangle adds w1 n_b + w2 n_c.  A
 // neighbour shared by two incident triangles appears twice in that sum with
-// the same weight; its record (8 bytes: vertex, position term) carries the
-// doubling in the sign bit, so that each neighbour is read once.  The sum
-// runs over the neighbours in vertex order (deterministic).
+// the same weight and is read once.  The sum runs over the neighbours in
+// vertex order (deterministic).
 // one neighbour's term, added to acc
 __device__ __forceinline__ void bilateral_add(float3& acc, uint2 e, float4 nb, float4 na, float sn2) {
   // the reference library is built with -use_fast_math (GMorpho/cuda.prf:47),
-  // so its exp and division here are the fast forms
+  // so its exp and division here are the fast forms.  Where neighbours nearly
+  // cancel, one rounding decides a normal's third digit: the sums are not
+  // fused and the division is not a product.
   float w = __expf(-__fadd_rn(__uint_as_float(e.y & 0x7fffffffu), __fdividef(dist2n(na, nb), sn2)));
   if (e.y >> 31) w = __fadd_rn(w, w);
   acc.x = __fadd_rn(acc.x, __fmul_rn(w, nb.x));
@@ -1071,21 +1036,28 @@ __device__ __forceinline__ float3 bilateral_sum(const float4* __restrict__ Nin, 
   return acc;
 }
 
-__global__ void k_bilateral(const float4* __restrict__ Nin, const uint32_t* __restrict__ roff,
-                            const uint2* __restrict__ rec, int64_t nv, float sn2, int zero_isolated,
-                            float4* __restrict__ Nout, float* __restrict__ N3) {
-  for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < nv; v += (int64_t)gridDim.x * blockDim.x) {
-    const uint32_t r0 = roff[v], n = roff[v + 1] - r0;
-    if (zero_isolated && n == 0) {
-      Nout[v] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (N3) { N3[3 * v] = 0.f; N3[3 * v + 1] = 0.f; N3[3 * v + 2] = 0.f; }
-      continue;
-    }
-    const float3 acc = bilateral_sum(Nin, rec + r0, n, Nin[v], sn2);
-    const float3 nn = normalize3(acc);
-    Nout[v] = make_float4(nn.x, nn.y, nn.z, 0.f);
-    if (N3) { N3[3 * v] = nn.x; N3[3 * v + 1] = nn.y; N3[3 * v + 2] = nn.z; }
+// one vertex of an iteration
+__device__ __forceinline__ void bilateral_vertex(const float4* __restrict__ Nin, const uint2* __restrict__ rec,
+                                                 const uint32_t* __restrict__ roff, uint32_t v, float sn2,
+                                                 int zero_isolated, float4* __restrict__ Nout,
+                                                 float* __restrict__ N3) {
+  const uint32_t at = roff_at(v), r0 = roff[at], n = roff[at + 1] - r0;
+  float3 nn = make_float3(0.f, 0.f, 0.f);
+  if (!(zero_isolated && n == 0)) nn = normalize3(bilateral_sum(Nin, rec + r0, n, Nin[v], sn2));
+  Nout[v] = make_float4(nn.x, nn.y, nn.z, 0.f);
+  if (N3) {
+    float* o = N3 + 3 * (size_t)v;
+    o[0] = nn.x; o[1] = nn.y; o[2] = nn.z;
   }
+}
+
+// (the 32 registers that keep eight blocks on an SM decide the time: 99 us for
+// 4.4M vertices; 115 to 118 at 44, spilled or not)
+__global__ void k_bilateral(const float4* __restrict__ Nin, const uint2* __restrict__ rec,
+                            const uint32_t* __restrict__ roff, uint32_t nv,
+                            float sn2, int zero_isolated, float4* __restrict__ Nout, float* __restrict__ N3) {
+  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += gridDim.x * blockDim.x)
+    bilateral_vertex(Nin, rec, roff, v, sn2, zero_isolated, Nout, N3);
 }
 
 // The same iteration over the vertices of several meshes at once (one
@@ -1094,8 +1066,8 @@ __global__ void k_bilateral(const float4* __restrict__ Nin, const uint32_t* __re
 struct BilMesh {
   const float4* Na;       // normals of even iterations' inputs (N4a)
   float4* Nb;             // and odd (N4b)
-  const uint32_t* roff;
   const uint2* rec;
+  const uint32_t* roff;
   float* N3;              // final normals (last iteration)
   int zero_isolated;
 };
@@ -1113,17 +1085,7 @@ __global__ void k_bilateral_group(const BilMesh* __restrict__ meshes, const int6
     const int64_t v = g - start[lo];
     const float4* Nin = odd ? M.Nb : M.Na;
     float4* Nout = odd ? const_cast<float4*>(M.Na) : M.Nb;
-    float* N3 = last ? M.N3 : nullptr;
-    const uint32_t r0 = M.roff[v], nrec = M.roff[v + 1] - r0;
-    if (M.zero_isolated && nrec == 0) {
-      Nout[v] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (N3) { N3[3 * v] = 0.f; N3[3 * v + 1] = 0.f; N3[3 * v + 2] = 0.f; }
-      continue;
-    }
-    const float3 acc = bilateral_sum(Nin, M.rec + r0, nrec, Nin[v], sn2);
-    const float3 nn = normalize3(acc);
-    Nout[v] = make_float4(nn.x, nn.y, nn.z, 0.f);
-    if (N3) { N3[3 * v] = nn.x; N3[3 * v + 1] = nn.y; N3[3 * v + 2] = nn.z; }
+    bilateral_vertex(Nin, M.rec, M.roff, (uint32_t)v, sn2, M.zero_isolated, Nout, last ? M.N3 : nullptr);
   }
 }
 
@@ -1152,8 +1114,8 @@ static int wave_blocks(const void* kernel, int64_t n, int sms) {
 }
 
 void MeshBuffers::release() {
-  cudaFree(V); cudaFree(N); cudaFree(N2); cudaFree(N4a); cudaFree(N4b); cudaFree(T); cudaFree(adj);
-  cudaFree(ent); cudaFree(rec); cudaFree(roff); cudaFree(rowptr); cudaFree(cursor); cudaFree(cell_voff); cudaFree(brick_tot);
+  cudaFree(V); cudaFree(N); cudaFree(N4a); cudaFree(N4b); cudaFree(T); cudaFree(adj); cudaFree(row0);
+  cudaFree(rec); cudaFree(roff); cudaFree(cursor); cudaFree(cell_voff); cudaFree(brick_tot);
   cudaFree(fix);
   *this = MeshBuffers();
 }
@@ -1213,21 +1175,20 @@ static cudaError_t ensure_grid_buffers(MeshBuffers& b, int64_t cells, int nb) {
 static cudaError_t ensure_vertex_buffers(MeshBuffers& b, int64_t nv) {
   cudaError_t e;
   if (b.v_cap < nv || b.V == nullptr) {
-    cudaFree(b.V); cudaFree(b.N); cudaFree(b.N4a); cudaFree(b.N4b); cudaFree(b.rowptr); cudaFree(b.cursor);
-    cudaFree(b.roff);
+    cudaFree(b.V); cudaFree(b.N); cudaFree(b.N4a); cudaFree(b.N4b); cudaFree(b.cursor);
+    cudaFree(b.adj); cudaFree(b.roff);
     b.V = b.N = nullptr;
     b.N4a = b.N4b = nullptr;
-    b.rowptr = b.cursor = nullptr;
-    b.roff = nullptr;
+    b.cursor = b.adj = b.roff = nullptr;
     b.v_cap = 0;
     const int64_t c = nv + nv / 4 + 1024;
     if ((e = cudaMalloc(&b.V, sizeof(float) * 3 * (size_t)c)) != cudaSuccess) return e;
     if ((e = cudaMalloc(&b.N, sizeof(float) * 3 * (size_t)c)) != cudaSuccess) return e;
     if ((e = cudaMalloc(&b.N4a, sizeof(float4) * (size_t)c)) != cudaSuccess) return e;
     if ((e = cudaMalloc(&b.N4b, sizeof(float4) * (size_t)c)) != cudaSuccess) return e;
-    if ((e = cudaMalloc(&b.rowptr, sizeof(uint32_t) * ((size_t)c + 1))) != cudaSuccess) return e;
-    if ((e = cudaMalloc(&b.cursor, sizeof(uint32_t) * ((size_t)c + 1))) != cudaSuccess) return e;
-    if ((e = cudaMalloc(&b.roff, sizeof(uint32_t) * ((size_t)c + 1))) != cudaSuccess) return e;
+    if ((e = cudaMalloc(&b.cursor, sizeof(uint32_t) * ((size_t)c + kCntWords))) != cudaSuccess) return e;
+    if ((e = cudaMalloc(&b.adj, sizeof(uint32_t) * kAdjMax * (size_t)c)) != cudaSuccess) return e;
+    if ((e = cudaMalloc(&b.roff, sizeof(uint32_t) * ((size_t)c + (size_t)c / kRecChunk + 4))) != cudaSuccess) return e;
     b.v_cap = c;
   }
   return cudaSuccess;
@@ -1236,14 +1197,13 @@ static cudaError_t ensure_vertex_buffers(MeshBuffers& b, int64_t nv) {
 static cudaError_t ensure_triangle_buffers(MeshBuffers& b, int64_t nt) {
   cudaError_t e;
   if (b.t_cap < nt || b.T == nullptr) {
-    cudaFree(b.T); cudaFree(b.adj); cudaFree(b.ent); cudaFree(b.rec);
-    b.T = b.adj = nullptr;
-    b.ent = b.rec = nullptr;
+    cudaFree(b.T); cudaFree(b.row0); cudaFree(b.rec);
+    b.T = b.row0 = nullptr;
+    b.rec = nullptr;
     b.t_cap = 0;
     const int64_t c = nt + nt / 4 + 1024;
     if ((e = cudaMalloc(&b.T, sizeof(uint32_t) * 3 * (size_t)c)) != cudaSuccess) return e;
-    if ((e = cudaMalloc(&b.adj, sizeof(uint32_t) * 3 * (size_t)c)) != cudaSuccess) return e;
-    if ((e = cudaMalloc(&b.ent, sizeof(uint2) * 6 * (size_t)c)) != cudaSuccess) return e;
+    if ((e = cudaMalloc(&b.row0, sizeof(uint32_t) * 3 * (size_t)c)) != cudaSuccess) return e;
     if ((e = cudaMalloc(&b.rec, sizeof(uint2) * 6 * (size_t)c)) != cudaSuccess) return e;
     b.t_cap = c;
   }
@@ -1333,38 +1293,22 @@ cudaError_t mesh_emit(const MeshArgs& a, MeshBuffers& b, int64_t nv, int64_t nt,
   if (nv == 0 || nt == 0) return cudaGetLastError();
   // normals
   const int sms = a.num_sms;
-  const int nchunks = (int)((nv + kScanChunk - 1) / kScanChunk);
-  const int nchunks0 = (int)((3 * nt + kRow0Chunk - 1) / kRow0Chunk);
-  // chunk sums (rows, then row 0) go to the per-cell offsets buffer, unused
-  // once the triangles are out
-  if ((int64_t)nchunks + nchunks0 + 2 > b.cells_cap) return cudaErrorInvalidValue;
-  uint32_t* sums = b.cell_voff;
-  uint32_t* offs0 = b.cell_voff + nchunks + 1;
-  cudaMemsetAsync(b.cursor, 0, sizeof(uint32_t) * (size_t)(nv + 1), st);
-  GM_LAUNCH(kc, "k_adj_count", st, k_adj_count<<<gs_blocks(3 * nt, 256, sms), 256, 0, st>>>(b.T, nt, b.cursor));
-  GM_LAUNCH(kc, "k_row0_count", st, k_row0_count<<<nchunks0, 256, 0, st>>>(b.T, 3 * nt, offs0));
-  GM_LAUNCH(kc, "k_scan_small", st, k_scan_small<<<1, 1024, 0, st>>>(offs0, nchunks0));
-  GM_LAUNCH(kc, "k_row0_total", st, k_row0_total<<<1, 32, 0, st>>>(offs0, nchunks0, b.cursor));
-  GM_LAUNCH(kc, "k_scan_sums", st, k_scan_sums<<<nchunks, 256, 0, st>>>(b.cursor, nv, sums));
-  GM_LAUNCH(kc, "k_scan_small", st, k_scan_small<<<1, 1024, 0, st>>>(sums, nchunks));
-  GM_LAUNCH(kc, "k_scan_apply", st, k_scan_apply<<<nchunks, 256, 0, st>>>(b.cursor, nv, sums, b.rowptr));
-  cudaMemsetAsync(b.cursor, 0, sizeof(uint32_t) * (size_t)(nv + 1), st);
-  GM_LAUNCH(kc, "k_adj_fill", st, k_adj_fill<<<gs_blocks(3 * nt, 256, sms), 256, 0, st>>>(b.T, nt, b.rowptr, b.cursor, b.adj));
-  GM_LAUNCH(kc, "k_row0_fill", st, k_row0_fill<<<nchunks0, 256, 0, st>>>(b.T, 3 * nt, offs0, b.rowptr, b.adj));
+  uint32_t* adj_more = b.adj + (size_t)kAdjRow * b.v_cap;
+  uint32_t* counters = b.cursor + nv;
   const int iters = a.bilateral_iters;
   const int zi = a.zero_isolated;
+  uint2* rec = iters > 0 ? b.rec : nullptr;
+  float* n3 = iters == 0 ? b.N : nullptr;
+  cudaMemsetAsync(b.cursor, 0, sizeof(uint32_t) * (size_t)(nv + kCntWords), st);
+  GM_LAUNCH(kc, "k_adj_slots", st,
+            k_adj_slots<<<gs_blocks(3 * nt, 256, sms), 256, 0, st>>>(b.T, nt, b.cursor, b.adj, adj_more));
+  GM_LAUNCH(kc, "k_row0_collect", st,
+            k_row0_collect<<<gs_blocks(3 * nt, 256, sms), 256, 0, st>>>(b.T, nt, b.cursor, counters, b.row0));
   GM_LAUNCH(kc, "k_adj_finish", st,
-            k_adj_finish<<<gs_blocks(nv, 256, sms), 256, 0, st>>>(b.V, b.T, b.rowptr, b.adj, nv, zi, b.N4a,
-                                                                  iters == 0 ? b.N : nullptr,
-                                                                  iters > 0 ? b.ent : nullptr, b.cursor));
-  if (iters > 0) {
-    // the records packed: counts (in cursor) scanned into roff
-    GM_LAUNCH(kc, "k_scan_sums", st, k_scan_sums<<<nchunks, 256, 0, st>>>(b.cursor, nv, sums));
-    GM_LAUNCH(kc, "k_scan_small", st, k_scan_small<<<1, 1024, 0, st>>>(sums, nchunks));
-    GM_LAUNCH(kc, "k_scan_apply", st, k_scan_apply<<<nchunks, 256, 0, st>>>(b.cursor, nv, sums, b.roff));
-    GM_LAUNCH(kc, "k_rec_pack", st,
-              k_rec_pack<<<gs_blocks(nv, 256, sms), 256, 0, st>>>(b.ent, b.rowptr, b.roff, nv, b.rec));
-  }
+            k_adj_finish<<<(unsigned)((nv + kRecChunk - 1) / kRecChunk), kRecChunk, 0, st>>>(
+                b.V, b.T, b.cursor, b.adj, adj_more, nv, zi, b.N4a, n3, rec, b.roff, counters));
+  GM_LAUNCH(kc, "k_row0_finish", st,
+            k_row0_finish<<<1, 1024, 0, st>>>(b.V, b.T, b.cursor, b.row0, nt, b.N4a, n3, rec, b.roff));
   if (a.defer_filter) return cudaGetLastError();
   float4* nin = b.N4a;
   float4* nout = b.N4b;
@@ -1372,8 +1316,8 @@ cudaError_t mesh_emit(const MeshArgs& a, MeshBuffers& b, int64_t nv, int64_t nt,
   for (int it = 0; it < iters; it++) {
     const float sn = it < 2 ? 1e10f : 0.2f;  // GMorpho.cu:6959-6969
     GM_LAUNCH(kc, "k_bilateral", st,
-              k_bilateral<<<bil_blocks, 256, 0, st>>>(nin, b.roff, b.rec, nv, sn * sn, zi, nout,
-                                                                   it == iters - 1 ? b.N : nullptr));
+              k_bilateral<<<bil_blocks, 256, 0, st>>>(nin, b.rec, b.roff, (uint32_t)nv, sn * sn, zi, nout,
+                                                      it == iters - 1 ? b.N : nullptr));
     float4* t = nin; nin = nout; nout = t;
   }
   return cudaGetLastError();
@@ -1391,7 +1335,7 @@ cudaError_t mesh_filter_group(MeshBuffers* const* meshes, const int64_t* nv, con
   hs[0] = 0;
   for (int i = 0; i < n; i++) {
     const MeshBuffers& b = *meshes[i];
-    hm[i] = BilMesh{b.N4a, b.N4b, b.roff, b.rec, b.N, zero_isolated[i]};
+    hm[i] = BilMesh{b.N4a, b.N4b, b.rec, b.roff, b.N, zero_isolated[i]};
     hs[i + 1] = hs[i] + nv[i];
   }
   const int64_t total = hs[n];
