@@ -272,8 +272,11 @@ struct MeshBuffers {
   uint32_t* cursor = nullptr;  // v_cap corner counts, then the mesh's counters
   int64_t v_cap = 0, t_cap = 0;
   // per-cell / per-brick scratch
-  uint32_t* cell_voff = nullptr;  // res^3
-  uint32_t* brick_tot = nullptr;  // 3 * (bricks + 1)
+  uint2* cells = nullptr;         // res^3: a mixed cell's corner block and first vertex
+  uint32_t* brick_tot = nullptr;  // 4 * (bricks + 1), then the scan's sums
+  uint32_t* brick_mask = nullptr; // 128 * bricks: a brick's mixed cells in Morton order
+  uint4* entries = nullptr;       // entries_cap: the mesh's mixed cells
+  int64_t entries_cap = 0, n_cells = 0;
   uint32_t* fix = nullptr;        // case-91 fix list: 1 + 4 * fix_cap
   int64_t cells_cap = 0, bricks_cap = 0;
   int fix_cap = 0;

@@ -20,20 +20,39 @@
 
 namespace gm {
 
-__constant__ uint64_t c_tri_packed[256] = GM_MC_TRI_PACKED_INIT;
-__constant__ uint8_t c_tri_count[256] = GM_MC_TRI_COUNT_INIT;
-__constant__ uint8_t c_tri_len[256] = GM_MC_TRI_LEN_INIT;
+// (global, not constant memory: the lanes of a warp read different entries)
+__device__ const uint64_t d_tri_packed[256] = GM_MC_TRI_PACKED_INIT;
+__device__ const uint8_t d_tri_count[256] = GM_MC_TRI_COUNT_INIT;
+__device__ const uint8_t d_tri_len[256] = GM_MC_TRI_LEN_INIT;
 
-// Edge mask of an MC cube value, derived from the corner order v0..v7 =
-// 000,100,110,010,001,101,111,011 and the edge list (0,1)(1,2)(2,3)(3,0)
-// (4,5)(5,6)(6,7)(7,4)(0,4)(1,5)(2,6)(3,7).
-__device__ __forceinline__ int edge_mask(int v) {
-  const int x = v ^ (v >> 1);
-  const int e3 = (v ^ (v >> 3)) & 1;
-  const int e7 = ((v >> 7) ^ (v >> 4)) & 1;
-  return (x & 7) | (e3 << 3) | (((x >> 4) & 7) << 4) | (e7 << 7) | (((v ^ (v >> 4)) & 0xF) << 8);
+// A cell's corner block: the occupancy of the 3^3 fine voxels at 2c + (i, j,
+// k), bit i + 3 j + 9 k, from which everything about its eight sub-cubes
+// follows by shifts: cube k (child order) has its corner at one of the eight
+// positions kCubes, corner bits at +0, 1, 4, 3, 9, 10, 13, 12
+// (ComputeMCMData, GMorpho.cu:6146-6232), and crossed edges 0, 3, 8 where
+// the bits at +1, +3, +9 differ.
+constexpr uint32_t kCubes = 0x361bu;  // positions 0, 1, 3, 4, 9, 10, 12, 13
+
+__device__ __forceinline__ uint32_t mixed_cubes(uint32_t b) {
+  uint32_t o = b | (b >> 1), a = b & (b >> 1);
+  o |= o >> 3, a &= a >> 3;
+  o |= o >> 9, a &= a >> 9;
+  return o & ~a & kCubes;
 }
-__device__ __forceinline__ int nv_owned(int em) { return (em & 1) + ((em >> 3) & 1) + ((em >> 8) & 1); }
+// crossed owned edges by cube position (a cube with one is mixed)
+__device__ __forceinline__ uint32_t edges0(uint32_t b) { return (b ^ (b >> 1)) & kCubes; }
+__device__ __forceinline__ uint32_t edges3(uint32_t b) { return (b ^ (b >> 3)) & kCubes; }
+__device__ __forceinline__ uint32_t edges8(uint32_t b) { return (b ^ (b >> 9)) & kCubes; }
+__device__ __forceinline__ int owned_vertices(uint32_t b) {
+  return __popc(edges0(b)) + __popc(edges3(b)) + __popc(edges8(b));
+}
+// the MC value of the cube at position p
+__device__ __forceinline__ uint32_t cube_value(uint32_t b, int p) {
+  const uint32_t x = b >> p;
+  return (x & 3u) | ((x >> 2) & 4u) | (x & 8u) | ((x >> 5) & 0x30u) | ((x >> 7) & 0x40u) | ((x >> 5) & 0x80u);
+}
+// position of the cube at (x, y, z) of its cell, each 0 or 1
+__device__ __forceinline__ int cube_pos(int x, int y, int z) { return x + 3 * y + 9 * z; }
 
 constexpr int kBrick = 16;               // cells per brick edge
 constexpr int kTileE = kBrick + 2;       // tile edge (halo 2 for neighbour cells)
@@ -90,64 +109,24 @@ __device__ bool load_tile_mixed(const uint8_t* __restrict__ C, GDims d, int ox, 
   return __syncthreads_or(seen0) && __syncthreads_or(seen1);
 }
 
-// The eight MC cube values of cell (local lx,ly,lz): cube k has its min
-// corner at fine voxel 2c + o_k; value bit j = occupancy of corner j
-// (ComputeMCMData, GMorpho.cu:6146-6232).
-__device__ __forceinline__ void cube_values(const uint8_t* tile, int lx, int ly, int lz, int vals[8]) {
-  uint32_t b27 = 0;
-#pragma unroll
-  for (int k = 0; k < 3; k++)
-#pragma unroll
-    for (int j = 0; j < 3; j++)
-#pragma unroll
-      for (int i = 0; i < 3; i++) {
-        const uint8_t cell = tile[tix(lx + (i >> 1), ly + (j >> 1), lz + (k >> 1))];
-        const uint32_t bit = (cell >> ((i & 1) + 2 * (j & 1) + 4 * (k & 1))) & 1u;
-        b27 |= bit << (i + 3 * j + 9 * k);
-      }
-#pragma unroll
-  for (int s = 0; s < 8; s++) {
-    const int ox = s & 1, oy = (s >> 1) & 1, oz = s >> 2;
-    const int b = ox + 3 * oy + 9 * oz;
-    // corners 000,100,110,010,001,101,111,011 -> offsets in the 27-cube
-    int v = 0;
-    v |= ((b27 >> (b + 0)) & 1) << 0;
-    v |= ((b27 >> (b + 1)) & 1) << 1;
-    v |= ((b27 >> (b + 4)) & 1) << 2;
-    v |= ((b27 >> (b + 3)) & 1) << 3;
-    v |= ((b27 >> (b + 9)) & 1) << 4;
-    v |= ((b27 >> (b + 10)) & 1) << 5;
-    v |= ((b27 >> (b + 13)) & 1) << 6;
-    v |= ((b27 >> (b + 12)) & 1) << 7;
-    vals[s] = v;
-  }
-}
-
-// The MC value of sub-cube s of cell (lx, ly, lz) alone (cube_values()[s]).
-__device__ __forceinline__ int cube_value(const uint8_t* tile, int lx, int ly, int lz, int s) {
-  const int fx = 2 * lx + (s & 1), fy = 2 * ly + ((s >> 1) & 1), fz = 2 * lz + (s >> 2);
-  int v = 0;
-#pragma unroll
-  for (int c = 0; c < 8; c++) {
-    // corners 000, 100, 110, 010, 001, 101, 111, 011
-    const int x = fx + (((c + 1) >> 1) & 1), y = fy + ((c >> 1) & 1), z = fz + (c >> 2);
-    const uint32_t cell = tile[tix(x >> 1, y >> 1, z >> 1)];
-    v |= (int)((cell >> ((x & 1) + 2 * (y & 1) + 4 * (z & 1))) & 1u) << c;
-  }
-  return v;
-}
-
-// True when the 2x2x2 block of cells c .. c+1 is all empty or all full: then
-// none of the eight sub-cubes of c is mixed (cheap test before cube_values).
-__device__ __forceinline__ bool cell_uniform(const uint8_t* tile, int lx, int ly, int lz) {
-  uint32_t o = 0, a = 0xffu;
-#pragma unroll
-  for (int k = 0; k < 8; k++) {
-    const uint32_t v = tile[tix(lx + (k & 1), ly + ((k >> 1) & 1), lz + (k >> 2))];
-    o |= v;
-    a &= v;
-  }
-  return o == 0u || a == 0xffu;
+// The corner block of tile cell (lx, ly, lz).
+__device__ __forceinline__ uint32_t corner_block(const uint8_t* tile, int lx, int ly, int lz) {
+  uint32_t c = tile[tix(lx, ly, lz)];
+  uint32_t b = (c & 3u) | ((c & 0xcu) << 1) | ((c & 0x30u) << 5) | ((c & 0xc0u) << 6);
+  c = tile[tix(lx + 1, ly, lz)];
+  b |= ((c & 1u) << 2) | ((c & 4u) << 3) | ((c & 0x10u) << 7) | ((c & 0x40u) << 8);
+  c = tile[tix(lx, ly + 1, lz)];
+  b |= ((c & 3u) << 6) | ((c & 0x30u) << 11);
+  c = tile[tix(lx + 1, ly + 1, lz)];
+  b |= ((c & 1u) << 8) | ((c & 0x10u) << 13);
+  c = tile[tix(lx, ly, lz + 1)];
+  b |= ((c & 3u) << 18) | ((c & 0xcu) << 19);
+  c = tile[tix(lx + 1, ly, lz + 1)];
+  b |= ((c & 1u) << 20) | ((c & 4u) << 21);
+  c = tile[tix(lx, ly + 1, lz + 1)];
+  b |= (c & 3u) << 24;
+  c = tile[tix(lx + 1, ly + 1, lz + 1)];
+  return b | ((c & 1u) << 26);
 }
 
 // Tagging / emission window of one meshing run.  A whole grid is its own
@@ -180,67 +159,10 @@ __device__ __forceinline__ bool brick_live(const McWin& w, int ox, int oy, int o
          oz + kBrick > w.tlo[2];
 }
 
-// mixed-cube mask of a cell (0 when the cell is not tagged)
-__device__ __forceinline__ int mixed_mask(const int vals[8], bool tagged) {
-  if (!tagged) return 0;
-  int m = 0;
-#pragma unroll
-  for (int s = 0; s < 8; s++) m |= (vals[s] != 0 && vals[s] != 255) ? (1 << s) : 0;
-  return m;
-}
-
-struct CellCounts {
-  uint32_t cubes, verts, tris, n91;
-};
-
-__device__ __forceinline__ CellCounts cell_counts(const int vals[8], int mask) {
-  CellCounts c{0, 0, 0, 0};
-#pragma unroll
-  for (int s = 0; s < 8; s++) {
-    if (!((mask >> s) & 1)) continue;
-    c.cubes += 1;
-    c.verts += nv_owned(edge_mask(vals[s]));
-    c.tris += c_tri_count[vals[s]];
-    c.n91 += c_tri_len[vals[s]] > c_tri_count[vals[s]] ? 1 : 0;
-  }
-  return c;
-}
-
 __device__ __forceinline__ void local_coords(int l, int& lx, int& ly, int& lz) {
   lx = (int)gather_bits3((uint32_t)l);
   ly = (int)gather_bits3((uint32_t)l >> 1);
   lz = (int)gather_bits3((uint32_t)l >> 2);
-}
-
-// block-wide exclusive scan of 4 counters (256 threads)
-__device__ __forceinline__ CellCounts block_exclusive_scan(CellCounts v, CellCounts& total) {
-  __shared__ uint32_t warp_tot[4][kMcThreads / 32];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  uint32_t a[4] = {v.cubes, v.verts, v.tris, v.n91};
-  uint32_t inc[4];
-#pragma unroll
-  for (int c = 0; c < 4; c++) {
-    uint32_t x = a[c];
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t t = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += t;
-    }
-    inc[c] = x;
-    if (lane == 31) warp_tot[c][wid] = x;
-  }
-  __syncthreads();
-  uint32_t wpre[4] = {0, 0, 0, 0}, tot[4] = {0, 0, 0, 0};
-#pragma unroll
-  for (int c = 0; c < 4; c++)
-    for (int w = 0; w < kMcThreads / 32; w++) {
-      if (w < wid) wpre[c] += warp_tot[c][w];
-      tot[c] += warp_tot[c][w];
-    }
-  __syncthreads();
-  total = CellCounts{tot[0], tot[1], tot[2], tot[3]};
-  return CellCounts{wpre[0] + inc[0] - a[0], wpre[1] + inc[1] - a[1], wpre[2] + inc[2] - a[2],
-                    wpre[3] + inc[3] - a[3]};
 }
 
 // block-wide exclusive scan of one counter (256 threads); total in `total`
@@ -266,62 +188,103 @@ __device__ __forceinline__ uint32_t block_scan1(uint32_t v, uint32_t& total) {
   return pre + x - v;
 }
 
-// The brick's own cells that may hold a tagged mixed cube (not uniform,
-// inside the tag window), in Morton order, into list[]; returns how many
-// (block-uniform).  The cube work then runs over this list with every lane
-// busy, instead of each thread walking its 16 cells and the warp taking the
-// slow path whenever one lane needs it.
-__device__ int brick_candidates(const uint8_t* tile, const McWin& w, int ox, int oy, int oz, uint16_t* list) {
-  uint32_t mask = 0;
-#pragma unroll 4
-  for (int i = 0; i < kCellsPerThread; i++) {
-    const int l = threadIdx.x * kCellsPerThread + i;
-    int lx, ly, lz;
-    local_coords(l, lx, ly, lz);
-    if (!cell_uniform(tile, lx, ly, lz) && win_tag(w, ox + lx, oy + ly, oz + lz)) mask |= 1u << i;
+// Cells of one row of a tile that may hold a tagged mixed cube (bit x): those
+// whose 2x2x2 block of cells is neither all empty nor all full, four at a
+// time as bytes of a word, inside the tag window.
+__device__ __forceinline__ uint32_t row_candidates(const uint8_t* tile, const McWin& w, int ox, int oy, int oz, int ly,
+                                                   int lz) {
+  const int gy = oy + ly + w.off[1], gz = oz + lz + w.off[2];
+  if (gy < 1 || gz < 1 || gy > w.gdim[1] - 2 || gz > w.gdim[2] - 2 || oy + ly < w.tlo[1] || oz + lz < w.tlo[2] ||
+      oy + ly >= w.thi[1] || oz + lz >= w.thi[2])
+    return 0u;
+  uint32_t o[5] = {0u, 0u, 0u, 0u, 0u}, a[5] = {~0u, ~0u, ~0u, ~0u, ~0u};
+#pragma unroll
+  for (int r = 0; r < 4; r++) {
+    const uint8_t* row = tile + tix(0, ly + (r & 1), lz + (r >> 1));
+    const uint4 q = *reinterpret_cast<const uint4*>(row);
+    const uint32_t h = *reinterpret_cast<const uint16_t*>(row + kBrick);
+    const uint32_t v[5] = {q.x, q.y, q.z, q.w, h};
+#pragma unroll
+    for (int j = 0; j < 5; j++) o[j] |= v[j], a[j] &= v[j];
   }
-  uint32_t total;
-  uint32_t k = block_scan1(__popc(mask), total);
-  while (mask) {
-    const int i = __ffs(mask) - 1;
-    mask &= mask - 1;
-    list[k++] = (uint16_t)(threadIdx.x * kCellsPerThread + i);
+  uint32_t cand = 0;
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    const uint32_t on = o[j] | (o[j] >> 8) | (o[j + 1] << 24), an = a[j] & ((a[j] >> 8) | (a[j + 1] << 24));
+    const uint32_t uniform = __vcmpeq4(on, 0u) | __vcmpeq4(an, 0xffffffffu);
+    cand |= (((~uniform & 0x08040201u) * 0x01010101u) >> 24) << (4 * j);
   }
-  __syncthreads();
-  return (int)total;
+  const int lo = max(max(1 - w.off[0], w.tlo[0]) - ox, 0), hi = min(min(w.gdim[0] - 1 - w.off[0], w.thi[0]) - ox, kBrick);
+  return hi <= lo ? 0u : cand & ((1u << hi) - (1u << lo));
 }
 
-__global__ void __launch_bounds__(kMcThreads, 5) k_mc_count(const uint8_t* __restrict__ C, GDims gd, McWin w,
-                                                          uint32_t* __restrict__ brick_tot) {
+// Counting pass, a block per brick: the mixed cells' corner blocks go to
+// cells[].x (where their cell lies: later passes and neighbours find them
+// there) and the brick's mask of them, in Morton order, to brick_mask, so
+// that the tile is read once per mesh; totals of mixed cells, vertices,
+// triangles and case-91 cubes to brick_tot.  At 1024^3 (4.4M vertices) 0.145
+// ms, bound by its tile loads and barriers; 0.264 when every cell was tested
+// byte by byte and its cubes built corner by corner.
+constexpr int kMaskWords = kCellsPerBrick / 32;
+__global__ void __launch_bounds__(kMcThreads, 6) k_mc_count(const uint8_t* __restrict__ C, GDims gd, McWin w,
+                                                          uint32_t* __restrict__ brick_tot,
+                                                          uint32_t* __restrict__ brick_mask, uint2* __restrict__ cells) {
   __shared__ __align__(16) uint8_t tile[kTileCells];
   __shared__ uint16_t list[kCellsPerBrick];
+  __shared__ uint32_t mask[kMaskWords], tot[4];
+  __shared__ uint8_t tab[256];  // triangles of a value, bit 7: one more than its slots (case 91)
   int ox, oy, oz;
   brick_origin(blockIdx.x, ox, oy, oz);
+  if (threadIdx.x < 4) tot[threadIdx.x] = 0u;
+  if (threadIdx.x < kMaskWords) mask[threadIdx.x] = 0u;
   if (!brick_live(w, ox, oy, oz) || !load_tile_mixed(C, gd, ox, oy, oz, tile)) {
-    if (threadIdx.x < 4) brick_tot[4 * blockIdx.x + threadIdx.x] = 0;
+    if (threadIdx.x < 4) brick_tot[4 * (size_t)blockIdx.x + threadIdx.x] = 0;
     return;
   }
-  const int nc = brick_candidates(tile, w, ox, oy, oz, list);
-  CellCounts acc{0, 0, 0, 0};
-  for (int j = threadIdx.x; j < nc; j += blockDim.x) {
-    int lx, ly, lz;
-    local_coords(list[j], lx, ly, lz);
-    int vals[8];
-    cube_values(tile, lx, ly, lz, vals);
-    const int m = mixed_mask(vals, true);
+  {
+    const uint32_t n = d_tri_count[threadIdx.x];
+    tab[threadIdx.x] = (uint8_t)(n | (d_tri_len[threadIdx.x] > n ? 0x80u : 0u));
+  }
+  const int ly = threadIdx.x & 15, lz = threadIdx.x >> 4;
+  uint32_t cand = row_candidates(tile, w, ox, oy, oz, ly, lz), nc;
+  uint32_t k = block_scan1(__popc(cand), nc);
+  while (cand) {
+    list[k++] = (uint16_t)((__ffs(cand) - 1) | (ly << 4) | (lz << 8));
+    cand &= cand - 1;
+  }
+  __syncthreads();
+  uint32_t n_cells = 0, n_verts = 0, n_tris = 0, n91 = 0;
+  for (uint32_t j = threadIdx.x; j < nc; j += kMcThreads) {
+    const int e = list[j], x = e & 15, y = (e >> 4) & 15, z = e >> 8;
+    const uint32_t b = corner_block(tile, x, y, z);
+    uint32_t m = mixed_cubes(b);
     if (!m) continue;
-    const CellCounts c = cell_counts(vals, m);
-    acc.cubes += c.cubes; acc.verts += c.verts;
-    if (win_emit(w, ox + lx, oy + ly, oz + lz)) { acc.tris += c.tris; acc.n91 += c.n91; }
+    cells[gidx(ox + x, oy + y, oz + z, gd)].x = b;
+    const uint32_t l = morton3((uint32_t)x, (uint32_t)y, (uint32_t)z);
+    atomicOr(mask + (l >> 5), 1u << (l & 31u));
+    n_cells++;
+    n_verts += owned_vertices(b);
+    if (!win_emit(w, ox + x, oy + y, oz + z)) continue;
+    while (m) {
+      const uint32_t t = tab[cube_value(b, __ffs(m) - 1)];
+      m &= m - 1;
+      n_tris += t & 7u;
+      n91 += t >> 7;
+    }
   }
-  CellCounts tot;
-  block_exclusive_scan(acc, tot);
-  if (threadIdx.x == 0) {
-    brick_tot[4 * blockIdx.x + 0] = tot.cubes;
-    brick_tot[4 * blockIdx.x + 1] = tot.verts;
-    brick_tot[4 * blockIdx.x + 2] = tot.tris;
-    brick_tot[4 * blockIdx.x + 3] = tot.n91;
+  n_cells = __reduce_add_sync(0xffffffffu, n_cells);
+  n_verts = __reduce_add_sync(0xffffffffu, n_verts);
+  n_tris = __reduce_add_sync(0xffffffffu, n_tris);
+  n91 = __reduce_add_sync(0xffffffffu, n91);
+  if ((threadIdx.x & 31) == 0 && n_cells) {
+    atomicAdd(tot + 0, n_cells);
+    atomicAdd(tot + 1, n_verts);
+    atomicAdd(tot + 2, n_tris);
+    atomicAdd(tot + 3, n91);
   }
+  __syncthreads();
+  if (threadIdx.x < 4) brick_tot[4 * (size_t)blockIdx.x + threadIdx.x] = tot[threadIdx.x];
+  if (tot[0] && threadIdx.x < kMaskWords) brick_mask[(size_t)blockIdx.x * kMaskWords + threadIdx.x] = mask[threadIdx.x];
 }
 
 // Exclusive scan of the four brick counters, in place, totals at index nb:
@@ -401,278 +364,215 @@ __device__ __forceinline__ float lerp_coord(float p1, float p2, float v1, float 
   return __fadd_rn(p1, __fsub_rn(v2, v1) > 0.f ? num : -num);
 }
 
-__global__ void __launch_bounds__(kMcThreads, 6) k_mc_vertices(const uint8_t* __restrict__ C, GDims gd, McWin w,
+// A mixed cell in Morton order: its brick and place (33 bits: the upper one
+// above the corner block's 27 bits), first vertex and first triangle.
+__device__ __forceinline__ uint4 pack_entry(uint32_t brick, uint32_t l, uint32_t b, uint32_t v, uint32_t t) {
+  return make_uint4((brick << 12) | l, b | ((brick >> 20) << 27), v, t);
+}
+
+// The mixed cells of a brick listed in Morton order (entries), each with its
+// first vertex and triangle from one scan per round of 256, and their
+// vertices.  A block per brick, from the counting pass's mask: no tile
+// (0.304 -> 0.090 ms at 1024^3).
+__global__ void __launch_bounds__(kMcThreads, 6) k_mc_vertices(GDims gd, McWin w,
                                                           const uint32_t* __restrict__ brick_off,
-                                                          uint32_t* __restrict__ cell_voff,
+                                                          const uint32_t* __restrict__ brick_mask,
+                                                          uint2* __restrict__ cells, uint4* __restrict__ entries,
                                                           float* __restrict__ V, float bx, float by, float bz,
                                                           float cs, float iso) {
-  __shared__ __align__(16) uint8_t tile[kTileCells];
   __shared__ uint16_t list[kCellsPerBrick];
+  __shared__ uint8_t tab[256];
+  const uint4 off = reinterpret_cast<const uint4*>(brick_off)[blockIdx.x];
+  const int nc = (int)(reinterpret_cast<const uint4*>(brick_off)[blockIdx.x + 1].x - off.x);
+  if (nc == 0) return;
   int ox, oy, oz;
   brick_origin(blockIdx.x, ox, oy, oz);
-  if (!brick_live(w, ox, oy, oz) || !load_tile_mixed(C, gd, ox, oy, oz, tile)) return;
-  const int nc = brick_candidates(tile, w, ox, oy, oz, list);
-  // the candidates in rounds of one per thread: a block scan of the round's
-  // vertex counts gives each its first vertex, in list (Morton) order
-  const uint32_t base = brick_off[4 * blockIdx.x + 1];
-  uint32_t run = 0;
+  tab[threadIdx.x] = d_tri_count[threadIdx.x];
+  {
+    // 16 cells a thread
+    uint32_t m = reinterpret_cast<const uint16_t*>(brick_mask + (size_t)blockIdx.x * kMaskWords)[threadIdx.x], n;
+    uint32_t k = block_scan1(__popc(m), n);
+    while (m) {
+      list[k++] = (uint16_t)(threadIdx.x * kCellsPerThread + __ffs(m) - 1);
+      m &= m - 1;
+    }
+  }
+  __syncthreads();
+  uint32_t run = 0;  // vertices and triangles of the rounds before (16 bits each a round, 32 in all)
+  uint32_t run_t = 0;
   for (int j0 = 0; j0 < nc; j0 += kMcThreads) {
     const int j = j0 + (int)threadIdx.x;
-    int lx = 0, ly = 0, lz = 0, m = 0;
-    int vals[8];
-    uint32_t nvert = 0;
+    uint32_t l = 0, b = 0, nv = 0, nt = 0;
+    int gx = 0, gy = 0, gz = 0;
+    int64_t g = 0;
     if (j < nc) {
-      local_coords(list[j], lx, ly, lz);
-      cube_values(tile, lx, ly, lz, vals);
-      m = mixed_mask(vals, true);
-      if (m) nvert = cell_counts(vals, m).verts;
+      l = list[j];
+      int lx, ly, lz;
+      local_coords((int)l, lx, ly, lz);
+      gx = ox + lx, gy = oy + ly, gz = oz + lz;
+      g = gidx(gx, gy, gz, gd);
+      b = cells[g].x;
+      nv = owned_vertices(b);
+      if (win_emit(w, gx, gy, gz))
+        for (uint32_t m = mixed_cubes(b); m; m &= m - 1) nt += tab[cube_value(b, __ffs(m) - 1)];
     }
-    uint32_t round_total;
-    const uint32_t pre = block_scan1(nvert, round_total);
-    const uint32_t first = base + run + pre;
-    run += round_total;
-    if (!m) continue;
-    const int gx = ox + lx, gy = oy + ly, gz = oz + lz;
-    uint32_t vo = first;
-    cell_voff[gidx(gx, gy, gz, gd)] = vo;
-    for (int s = 0; s < 8; s++) {
-      if (!((m >> s) & 1)) continue;
-      const int v = vals[s];
-      const int em = edge_mask(v);
+    uint32_t total;
+    const uint32_t pre = block_scan1(nv | (nt << 16), total);  // (at most 24 and 40 a cell)
+    uint32_t vo = off.y + run + (pre & 0xffffu);
+    const uint32_t to = off.z + run_t + (pre >> 16);
+    run += total & 0xffffu;
+    run_t += total >> 16;
+    if (j >= nc) continue;
+    entries[off.x + j] = pack_entry(blockIdx.x, l, b, vo, to);
+    cells[g].y = vo;
+    for (uint32_t own = edges0(b) | edges3(b) | edges8(b); own; own &= own - 1) {
+      const int p = __ffs(own) - 1, sz = p >= 9 ? 1 : 0, sy = p - 9 * sz >= 3 ? 1 : 0, sx = p - 9 * sz - 3 * sy;
+      const uint32_t c = b >> p;
       // corner point from GLOBAL fine coordinates, so that a crop's vertices
       // are bit-identical to the whole grid's
-      const int fx = 2 * (gx + w.off[0]) + (s & 1), fy = 2 * (gy + w.off[1]) + ((s >> 1) & 1),
-                fz = 2 * (gz + w.off[2]) + (s >> 2);
-      const float px = __fmaf_rn((float)fx, cs, bx);
-      const float py = __fmaf_rn((float)fy, cs, by);
-      const float pz = __fmaf_rn((float)fz, cs, bz);
-      const float v0 = (v & 1) ? 1.f : 0.f, v1 = (v & 2) ? 1.f : 0.f, v3 = (v & 8) ? 1.f : 0.f,
-                  v4 = (v & 16) ? 1.f : 0.f;
-      if (em & 1) {  // edge 0: point -> point + (cs,0,0)
-        float* o = V + 3 * (size_t)vo;
+      const float px = __fmaf_rn((float)(2 * (gx + w.off[0]) + sx), cs, bx);
+      const float py = __fmaf_rn((float)(2 * (gy + w.off[1]) + sy), cs, by);
+      const float pz = __fmaf_rn((float)(2 * (gz + w.off[2]) + sz), cs, bz);
+      const float v0 = (c & 1u) ? 1.f : 0.f, v1 = (c & 2u) ? 1.f : 0.f, v3 = (c & 8u) ? 1.f : 0.f,
+                  v4 = (c & 512u) ? 1.f : 0.f;
+      if (v0 != v1) {  // edge 0: point -> point + (cs,0,0)
+        float* o = V + 3 * (size_t)vo++;
         o[0] = lerp_coord(px, __fadd_rn(px, cs), v0, v1, iso);
         o[1] = lerp_coord(py, py, v0, v1, iso);
         o[2] = lerp_coord(pz, pz, v0, v1, iso);
-        vo++;
       }
-      if (em & 8) {  // edge 3: point + (0,cs,0) -> point
+      if (v0 != v3) {  // edge 3: point + (0,cs,0) -> point
         const float p1y = __fadd_rn(py, cs);
-        float* o = V + 3 * (size_t)vo;
+        float* o = V + 3 * (size_t)vo++;
         o[0] = lerp_coord(px, px, v3, v0, iso);
         o[1] = lerp_coord(p1y, py, v3, v0, iso);
         o[2] = lerp_coord(pz, pz, v3, v0, iso);
-        vo++;
       }
-      if (em & 256) {  // edge 8: point -> point + (0,0,cs)
-        float* o = V + 3 * (size_t)vo;
+      if (v0 != v4) {  // edge 8: point -> point + (0,0,cs)
+        float* o = V + 3 * (size_t)vo++;
         o[0] = lerp_coord(px, px, v0, v4, iso);
         o[1] = lerp_coord(py, py, v0, v4, iso);
         o[2] = lerp_coord(pz, __fadd_rn(pz, cs), v0, v4, iso);
-        vo++;
       }
     }
   }
 }
 
-// Per-cell summary used for neighbour lookups: bits 0..7 = mixed cubes,
-// bits 8+k / 16+k / 24+k = cube k owns a vertex on edge 0 / 3 / 8.
-__device__ __forceinline__ uint32_t cell_info(const uint8_t* tile, int lx, int ly, int lz, bool tagged) {
-  if (!tagged || cell_uniform(tile, lx, ly, lz)) return 0u;
-  int vals[8];
-  cube_values(tile, lx, ly, lz, vals);
-  const int m = mixed_mask(vals, true);
-  uint32_t info = (uint32_t)m;
-#pragma unroll
-  for (int s = 0; s < 8; s++) {
-    if (!((m >> s) & 1)) continue;
-    const int em = edge_mask(vals[s]);
-    info |= (uint32_t)(em & 1) << (8 + s);
-    info |= (uint32_t)((em >> 3) & 1) << (16 + s);
-    info |= (uint32_t)((em >> 8) & 1) << (24 + s);
-  }
-  return info;
-}
-
-constexpr int kInfoE = kBrick + 1;  // cells 0..16 of the brick (own + one neighbour layer)
-
-__device__ __forceinline__ uint32_t info_of(const int vals[8], int m) {
-  uint32_t info = (uint32_t)m;
-#pragma unroll
-  for (int s = 0; s < 8; s++) {
-    if (!((m >> s) & 1)) continue;
-    const int em = edge_mask(vals[s]);
-    info |= (uint32_t)(em & 1) << (8 + s);
-    info |= (uint32_t)((em >> 3) & 1) << (16 + s);
-    info |= (uint32_t)((em >> 8) & 1) << (24 + s);
-  }
-  return info;
-}
-
-// dynamic shared memory of k_mc_triangles
-constexpr size_t kTriSmem = sizeof(uint32_t) * kInfoE * kInfoE * kInfoE + sizeof(uint16_t) * kCellsPerBrick +
-                            sizeof(uint16_t) * 8 * kMcThreads + kTileCells;
-
-// Vertex offset of cube k of the cell whose summary is `info` (absent: -1),
-// with its edge-0 / edge-3 ownership.
-__device__ __forceinline__ long long cube_voff(uint32_t info, uint32_t cell_off, int k, int& e0, int& e3) {
-  if (!((info >> k) & 1)) { e0 = e3 = 0; return -1; }
-  const uint32_t below = info & ((1u << k) - 1u);
-  const uint32_t off = cell_off + __popc((info >> 8) & below) + __popc((info >> 16) & below) +
-                       __popc((info >> 24) & below);
-  e0 = (info >> (8 + k)) & 1;
-  e3 = (info >> (16 + k)) & 1;
-  return (long long)off;
-}
-
-__global__ void __launch_bounds__(kMcThreads, 5) k_mc_triangles(const uint8_t* __restrict__ C, GDims gd, McWin w,
-                                                              const uint32_t* __restrict__ brick_off,
-                                                              const uint32_t* __restrict__ cell_voff,
-                                                              uint32_t* __restrict__ T, uint32_t nt_total,
-                                                              uint32_t* __restrict__ fix, int fix_cap) {
-  extern __shared__ uint4 mc_smem[];
-  uint8_t* tile = reinterpret_cast<uint8_t*>(mc_smem);                          // [18 * 18 rows of kTileP]
-  uint32_t* info = reinterpret_cast<uint32_t*>(tile + kTileCells);              // [17^3]
-  uint16_t* list = reinterpret_cast<uint16_t*>(info + kInfoE * kInfoE * kInfoE);  // [4096]
-  int ox, oy, oz;
-  brick_origin(blockIdx.x, ox, oy, oz);
-  if (!brick_live(w, ox, oy, oz) || !load_tile_mixed(C, gd, ox, oy, oz, tile)) return;
-  for (int i = threadIdx.x; i < kInfoE * kInfoE * kInfoE; i += blockDim.x) info[i] = 0u;
-  const int nc = brick_candidates(tile, w, ox, oy, oz, list);
-  // summaries of the own candidates
-  for (int j = threadIdx.x; j < nc; j += blockDim.x) {
-    int lx, ly, lz;
-    local_coords(list[j], lx, ly, lz);
-    int vals[8];
-    cube_values(tile, lx, ly, lz, vals);
-    info[lx + kInfoE * (ly + kInfoE * lz)] = info_of(vals, mixed_mask(vals, true));
-  }
-  // the neighbour layer (cells 16 along some axis)
-  for (int i = threadIdx.x; i < kInfoE * kInfoE * kInfoE; i += blockDim.x) {
-    const int lx = i % kInfoE, ly = (i / kInfoE) % kInfoE, lz = i / (kInfoE * kInfoE);
-    if (lx < kBrick && ly < kBrick && lz < kBrick) continue;
-    info[i] = cell_info(tile, lx, ly, lz, win_tag(w, ox + lx, oy + ly, oz + lz));
+// Triangles: eight lanes per listed cell, one per sub-cube, over the whole
+// list (a small grid's bricks spread over all SMs).  Lane k also holds the
+// neighbour cell at offset k (corner block and first vertex): the cubes whose
+// edges a cube's triangles use lie in those eight cells, so their vertices
+// come by shuffles.  A neighbour outside the tag window has no vertices (its
+// edges take index 0); inside it, a crossed edge's owner is mixed, so its
+// words are this mesh's.  0.626 -> 0.214 ms at 1024^3, and 84 -> 11 us at
+// 128^3, where a block per brick (tile, summaries of 17^3 cells, rounds with
+// three barriers each) left most SMs idle.
+__global__ void __launch_bounds__(kMcThreads) k_mc_triangles(GDims gd, McWin w, const uint2* __restrict__ cells,
+                                                            const uint4* __restrict__ entries, uint32_t ncells,
+                                                            uint32_t* __restrict__ T, uint32_t nt_total,
+                                                            uint32_t* __restrict__ fix, int fix_cap) {
+  __shared__ uint64_t tab[256];             // edges of a value's triangles, its count in the upper bits
+  __shared__ uint32_t vert[12][kMcThreads];  // edge vertices of each thread's cube
+  {
+    const uint32_t n = d_tri_count[threadIdx.x];
+    tab[threadIdx.x] = d_tri_packed[threadIdx.x] | ((uint64_t)(n | (d_tri_len[threadIdx.x] > n ? 8u : 0u)) << 60);
   }
   __syncthreads();
-  // The candidates in rounds of one per thread; each round's mixed cubes
-  // (cell in list order, then sub-cube order) go to a cube list and are
-  // worked one per thread, a block scan of their triangle counts giving
-  // each its first triangle: the order of the cell-by-cell walk, without
-  // the lanes of a warp waiting on each other's sub-cube loops.
-  uint16_t* cubes = list + kCellsPerBrick;  // [8 * kMcThreads]: (cell slot << 3) | sub-cube
-  const uint32_t tbase = brick_off[4 * blockIdx.x + 2];
-  uint32_t run = 0;
-  for (int j0 = 0; j0 < nc; j0 += kMcThreads) {
-    const int j = j0 + (int)threadIdx.x;
-    uint32_t m = 0;
-    if (j < nc) {
-      int lx, ly, lz;
-      local_coords(list[j], lx, ly, lz);
-      m = info[lx + kInfoE * (ly + kInfoE * lz)] & 0xffu;
-      if (m != 0 && !win_emit(w, ox + lx, oy + ly, oz + lz)) m = 0;
-    }
-    uint32_t nround;
-    uint32_t k = block_scan1((uint32_t)__popc(m), nround);
-    while (m) {
-      const int sc = __ffs(m) - 1;
-      m &= m - 1;
-      cubes[k++] = (uint16_t)((threadIdx.x << 3) | sc);
-    }
-    __syncthreads();
-    for (int c0 = 0; c0 < (int)nround; c0 += kMcThreads) {
-      const int c = c0 + (int)threadIdx.x;
-      int lx = 0, ly = 0, lz = 0, s = 0, v = 0, cnt = 0;
-      if (c < (int)nround) {
-        const int e = cubes[c];
-        s = e & 7;
-        local_coords(list[j0 + (e >> 3)], lx, ly, lz);
-        v = cube_value(tile, lx, ly, lz, s);
-        cnt = c_tri_count[v];
+  const int lane = threadIdx.x & 31, k = lane & 7, kx = k & 1, ky = (k >> 1) & 1, kz = k >> 2;
+  // (the grid covers whole warps: all lanes of a warp run as many rounds)
+  const uint32_t stride = gridDim.x * (kMcThreads / 8);
+  for (uint32_t i0 = (blockIdx.x * kMcThreads + (threadIdx.x & ~31u)) / 8; i0 < ncells; i0 += stride) {
+    const uint32_t i = i0 + (lane >> 3);
+    uint4 e = make_uint4(0u, 0u, 0u, 0u);
+    int gx = 0, gy = 0, gz = 0;
+    uint32_t b = 0, nb = 0, nvo = 0;  // own block; the neighbour's block and first vertex
+    bool tagged = false, emit = false;
+    if (i < ncells) {
+      e = entries[i];
+      b = e.y & 0x7ffffffu;
+      const uint32_t brick = (e.x >> 12) | ((e.y >> 27) << 20);
+      int ox, oy, oz, lx, ly, lz;
+      brick_origin((int)brick, ox, oy, oz);
+      local_coords((int)(e.x & 0xfffu), lx, ly, lz);
+      gx = ox + lx, gy = oy + ly, gz = oz + lz;
+      emit = win_emit(w, gx, gy, gz);
+      const int x = gx + kx, y = gy + ky, z = gz + kz;
+      tagged = x < gd.x && y < gd.y && z < gd.z && win_tag(w, x, y, z);
+      if (k == 0) {
+        nb = b, nvo = e.z;
+      } else if (tagged && emit) {
+        const uint2 c = cells[gidx(x, y, z, gd)];
+        nb = c.x, nvo = c.y;
       }
-      uint32_t ttot;
-      const uint32_t pre = block_scan1((uint32_t)cnt, ttot);
-      const uint32_t to = tbase + run + pre;
-      run += ttot;
-      if (c >= (int)nround) continue;
-      const int gx = ox + lx, gy = oy + ly, gz = oz + lz;
-      const int em = edge_mask(v);
-      const int fx = 2 * gx + (s & 1), fy = 2 * gy + ((s >> 1) & 1), fz = 2 * gz + (s >> 2);  // local
-      int o0 = 0, o3 = 0;
-      const uint32_t vo = (uint32_t)cube_voff(info[lx + kInfoE * (ly + kInfoE * lz)],
-                                              cell_voff[gidx(gx, gy, gz, gd)], s, o0, o3);
-      uint32_t vert[12];
+    }
+    const uint32_t tags = __ballot_sync(0xffffffffu, tagged) >> (lane & 24);
+    const int p = cube_pos(kx, ky, kz);
+    const bool cube = emit && ((mixed_cubes(b) >> p) & 1u);
+    const uint32_t val = cube_value(b, p);
+    const uint64_t tl = tab[val];
+    const uint32_t cnt = cube ? (uint32_t)(tl >> 60) & 7u : 0u;
+    uint32_t incl = cnt;
 #pragma unroll
-      for (int e = 0; e < 12; e++) vert[e] = 0;
-      {
-        uint32_t ind = 0;
-        if (em & 1) vert[0] = vo + ind++;
-        if (em & 8) vert[3] = vo + ind++;
-        if (em & 256) vert[8] = vo + ind++;
-      }
-      // neighbour cubes +x, +x+y, +y, +z, +x+z, +y+z (BuildNeighbors order,
-      // GMorpho.cu:6480-6487) and the edges they own
-      // (MarchingCubesMesher.cu:1392-1456)
-      auto nb = [&](int dx, int dy, int dz, int& e0, int& e3) -> long long {
-        const int nfx = fx + dx, nfy = fy + dy, nfz = fz + dz;
-        const int cx = (nfx >> 1) - ox, cy = (nfy >> 1) - oy, cz = (nfz >> 1) - oz;
-        const uint32_t ninfo = info[cx + kInfoE * (cy + kInfoE * cz)];
-        const int kk = (nfx & 1) | ((nfy & 1) << 1) | ((nfz & 1) << 2);
-        if (!((ninfo >> kk) & 1)) { e0 = e3 = 0; return -1; }
-        return cube_voff(ninfo, cell_voff[gidx(nfx >> 1, nfy >> 1, nfz >> 1, gd)], kk, e0, e3);
-      };
-      int a0 = 0, a3 = 0;
-      if (em & (2 | 512)) {
-        const long long id1 = nb(1, 0, 0, a0, a3);
-        if ((em & 2) && id1 >= 0) vert[1] = (uint32_t)id1 + a0;
-        if (em & 512) vert[9] = id1 >= 0 ? (uint32_t)id1 + a0 + a3 : 0u;
-      }
-      if (em & 1024) {
-        const long long id2 = nb(1, 1, 0, a0, a3);
-        vert[10] = id2 >= 0 ? (uint32_t)id2 + a0 + a3 : 0u;
-      }
-      if (em & (4 | 2048)) {
-        const long long id3 = nb(0, 1, 0, a0, a3);
-        if (em & 4) vert[2] = id3 >= 0 ? (uint32_t)id3 : 0u;
-        if (em & 2048) vert[11] = id3 >= 0 ? (uint32_t)id3 + a0 + a3 : 0u;
-      }
-      if (em & (16 | 128)) {
-        const long long id4 = nb(0, 0, 1, a0, a3);
-        if (em & 16) vert[4] = id4 >= 0 ? (uint32_t)id4 : 0u;
-        if ((em & 128) && id4 >= 0) vert[7] = (uint32_t)id4 + a0;
-      }
-      if (em & 32) {
-        const long long id5 = nb(1, 0, 1, a0, a3);
-        if (id5 >= 0) vert[5] = (uint32_t)id5 + a0;
-      }
-      if (em & 64) {
-        const long long id7 = nb(0, 1, 1, a0, a3);
-        vert[6] = id7 >= 0 ? (uint32_t)id7 : 0u;
-      }
-      // reversed winding (MarchingCubesMesher.cu:1487-1497)
-      const uint64_t tl = c_tri_packed[v];
-      for (int t = 0; t < cnt; t++) {
-        uint32_t* o = T + 3 * (size_t)(to + t);
-        o[0] = vert[(tl >> (4 * (3 * t + 2))) & 0xf];
-        o[1] = vert[(tl >> (4 * (3 * t + 1))) & 0xf];
-        o[2] = vert[(tl >> (4 * (3 * t))) & 0xf];
-      }
-      if (c_tri_len[v] > cnt) {
-        // Case 91: the reference writes one more triangle than its slot
-        // count; it lands on the next slot (the next cube's first triangle)
-        // and, written later, wins; past the end it is dropped.
-        const uint32_t slot = to + cnt;
-        if (slot < nt_total) {
-          const int idx = (int)atomicAdd(fix, 1u);
-          if (idx < fix_cap) {
-            uint32_t* f = fix + 1 + 4 * idx;
-            f[0] = slot;
-            f[1] = vert[(tl >> (4 * (3 * cnt + 2))) & 0xf];
-            f[2] = vert[(tl >> (4 * (3 * cnt + 1))) & 0xf];
-            f[3] = vert[(tl >> (4 * (3 * cnt))) & 0xf];
-          }
+    for (int o = 1; o < 8; o <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o, 8);
+      if (k >= o) incl += t;
+    }
+    const uint32_t to = e.w + incl - cnt;
+    // crossed edges: 0 (0,1) 1 (1,2) 2 (2,3) 3 (3,0) 4 (4,5) 5 (5,6) 6 (6,7)
+    // 7 (7,4) 8 (0,4) 9 (1,5) 10 (2,6) 11 (3,7); their owner cubes are this
+    // one and those at +x, +x+y, +y, +z, +x+z, +y+z, their own edges 0, 3, 8
+    // (BuildNeighbors order, GMorpho.cu:6480-6487;
+    // MarchingCubesMesher.cu:1392-1456)
+    auto owner = [&](int dx, int dy, int dz, uint32_t& first, uint32_t& e0, uint32_t& e3) -> bool {
+      const int fx = kx + dx, fy = ky + dy, fz = kz + dz;
+      const int cell = (fx >> 1) | ((fy >> 1) << 1) | ((fz >> 1) << 2);
+      const uint32_t ob = __shfl_sync(0xffffffffu, nb, cell, 8), ov = __shfl_sync(0xffffffffu, nvo, cell, 8);
+      const int q = cube_pos(fx & 1, fy & 1, fz & 1);
+      const uint32_t below = (1u << q) - 1u, m0 = edges0(ob), m3 = edges3(ob), m8 = edges8(ob);
+      first = ov + __popc(m0 & below) + __popc(m3 & below) + __popc(m8 & below);
+      e0 = (m0 >> q) & 1u;
+      e3 = (m3 >> q) & 1u;
+      return (tags >> cell) & 1u;
+    };
+    uint32_t f, e0, e3;
+    uint32_t(*my)[kMcThreads] = reinterpret_cast<uint32_t(*)[kMcThreads]>(&vert[0][threadIdx.x]);
+    bool ok = owner(0, 0, 0, f, e0, e3);
+    my[0][0] = f, my[3][0] = f + e0, my[8][0] = f + e0 + e3;
+    ok = owner(1, 0, 0, f, e0, e3);
+    my[1][0] = ok ? f + e0 : 0u, my[9][0] = ok ? f + e0 + e3 : 0u;
+    ok = owner(1, 1, 0, f, e0, e3);
+    my[10][0] = ok ? f + e0 + e3 : 0u;
+    ok = owner(0, 1, 0, f, e0, e3);
+    my[2][0] = ok ? f : 0u, my[11][0] = ok ? f + e0 + e3 : 0u;
+    ok = owner(0, 0, 1, f, e0, e3);
+    my[4][0] = ok ? f : 0u, my[7][0] = ok ? f + e0 : 0u;
+    ok = owner(1, 0, 1, f, e0, e3);
+    my[5][0] = ok ? f + e0 : 0u;
+    ok = owner(0, 1, 1, f, e0, e3);
+    my[6][0] = ok ? f : 0u;
+    // reversed winding (MarchingCubesMesher.cu:1487-1497)
+    for (uint32_t t = 0; t < cnt; t++) {
+      uint32_t* o = T + 3 * (size_t)(to + t);
+      o[0] = my[(tl >> (4 * (3 * t + 2))) & 0xf][0];
+      o[1] = my[(tl >> (4 * (3 * t + 1))) & 0xf][0];
+      o[2] = my[(tl >> (4 * (3 * t))) & 0xf][0];
+    }
+    if (cube && (tl >> 63)) {
+      // Case 91: the reference writes one more triangle than its slot
+      // count; it lands on the next slot (the next cube's first triangle)
+      // and, written later, wins; past the end it is dropped.
+      const uint32_t slot = to + cnt;
+      if (slot < nt_total) {
+        const int idx = (int)atomicAdd(fix, 1u);
+        if (idx < fix_cap) {
+          uint32_t* o = fix + 1 + 4 * idx;
+          o[0] = slot;
+          o[1] = my[(tl >> (4 * (3 * cnt + 2))) & 0xf][0];
+          o[2] = my[(tl >> (4 * (3 * cnt + 1))) & 0xf][0];
+          o[3] = my[(tl >> (4 * (3 * cnt))) & 0xf][0];
         }
       }
     }
-    __syncthreads();  // the cube list is rewritten by the next round
   }
 }
 
@@ -1115,7 +1015,8 @@ static int wave_blocks(const void* kernel, int64_t n, int sms) {
 
 void MeshBuffers::release() {
   cudaFree(V); cudaFree(N); cudaFree(N4a); cudaFree(N4b); cudaFree(T); cudaFree(adj); cudaFree(row0);
-  cudaFree(rec); cudaFree(roff); cudaFree(cursor); cudaFree(cell_voff); cudaFree(brick_tot);
+  cudaFree(rec); cudaFree(roff); cudaFree(cursor); cudaFree(cells); cudaFree(brick_tot);
+  cudaFree(brick_mask); cudaFree(entries);
   cudaFree(fix);
   *this = MeshBuffers();
 }
@@ -1155,17 +1056,21 @@ static McWin window_of(const MeshArgs& a) {
 static cudaError_t ensure_grid_buffers(MeshBuffers& b, int64_t cells, int nb) {
   cudaError_t e;
   if (nb + 1 > b.bricks_cap) {
-    if (b.brick_tot) cudaFree(b.brick_tot);
-    b.brick_tot = nullptr;
+    cudaFree(b.brick_tot);
+    cudaFree(b.brick_mask);
+    b.brick_tot = b.brick_mask = nullptr;
+    b.bricks_cap = 0;
+    if ((e = cudaMalloc(&b.brick_mask, sizeof(uint32_t) * kMaskWords * (size_t)nb)) != cudaSuccess) return e;
     // counters and totals (nb + 1), then the chunk sums of the scan
     e = cudaMalloc(&b.brick_tot, sizeof(uint32_t) * 4 * ((size_t)nb + 1 + (nb + kBrickChunk - 1) / kBrickChunk));
     if (e != cudaSuccess) return e;
     b.bricks_cap = nb + 1;
   }
   if (cells > b.cells_cap) {
-    if (b.cell_voff) cudaFree(b.cell_voff);
-    b.cell_voff = nullptr;
-    e = cudaMalloc(&b.cell_voff, sizeof(uint32_t) * (size_t)cells);
+    cudaFree(b.cells);
+    b.cells = nullptr;
+    b.cells_cap = 0;
+    e = cudaMalloc(&b.cells, sizeof(uint2) * (size_t)cells);
     if (e != cudaSuccess) return e;
     b.cells_cap = cells;
   }
@@ -1210,11 +1115,23 @@ static cudaError_t ensure_triangle_buffers(MeshBuffers& b, int64_t nt) {
   return cudaSuccess;
 }
 
+static cudaError_t ensure_entries(MeshBuffers& b, int64_t n) {
+  if (b.entries_cap >= n && b.entries != nullptr) return cudaSuccess;
+  cudaFree(b.entries);
+  b.entries = nullptr;
+  b.entries_cap = 0;
+  const int64_t c = n + n / 4 + 1024;
+  const cudaError_t e = cudaMalloc(&b.entries, sizeof(uint4) * (size_t)c);
+  if (e == cudaSuccess) b.entries_cap = c;
+  return e;
+}
+
 cudaError_t mesh_reserve(MeshBuffers& b, int res, int64_t nv, int64_t nt) {
   const int d[3] = {res, res, res};
   cudaError_t e = ensure_grid_buffers(b, (int64_t)res * res * res, brick_count(d));
   if (e == cudaSuccess) e = ensure_vertex_buffers(b, nv);
   if (e == cudaSuccess) e = ensure_triangle_buffers(b, nt);
+  if (e == cudaSuccess) e = ensure_entries(b, nv + nv / 2);
   return e;
 }
 
@@ -1227,7 +1144,8 @@ cudaError_t mesh_count_launch(const MeshArgs& a, MeshBuffers& b, cudaStream_t st
   const int nb = brick_count(d);
   cudaError_t e = ensure_grid_buffers(b, cells, nb);
   if (e != cudaSuccess) return e;
-  GM_LAUNCH(kc, "k_mc_count", st, k_mc_count<<<nb, kMcThreads, 0, st>>>(a.C, gd, window_of(a), b.brick_tot));
+  GM_LAUNCH(kc, "k_mc_count", st, k_mc_count<<<nb, kMcThreads, 0, st>>>(a.C, gd, window_of(a), b.brick_tot,
+                                                                          b.brick_mask, b.cells));
   {
     const int nchunks = (nb + kBrickChunk - 1) / kBrickChunk;
     if (nchunks > kBrickChunk) return cudaErrorInvalidValue;
@@ -1244,6 +1162,7 @@ cudaError_t mesh_prepare_grid(const MeshArgs& a, MeshBuffers& b) {
 }
 
 cudaError_t mesh_count_finish(MeshBuffers& b, const uint32_t* tot, int64_t* nv, int64_t* nt) {
+  b.n_cells = tot[0];
   *nv = tot[1];
   *nt = tot[2];
   const int need_fix = (int)tot[3];
@@ -1283,11 +1202,14 @@ cudaError_t mesh_emit(const MeshArgs& a, MeshBuffers& b, int64_t nv, int64_t nt,
   if ((e = ensure_triangle_buffers(b, nt)) != cudaSuccess) return e;
   const float cs = 0.5f * a.cell_size;  // exact: scaling by a power of two
   cudaMemsetAsync(b.fix, 0, sizeof(uint32_t), st);
-  GM_LAUNCH(kc, "k_mc_vertices", st, k_mc_vertices<<<nb, kMcThreads, 0, st>>>(a.C, gd, w, b.brick_tot, b.cell_voff, b.V, a.bbox_min[0], a.bbox_min[1],
-                                           a.bbox_min[2], cs, a.isovalue));
-  ensure_dynamic_smem(reinterpret_cast<const void*>(k_mc_triangles), kTriSmem);
-  GM_LAUNCH(kc, "k_mc_triangles", st, k_mc_triangles<<<nb, kMcThreads, kTriSmem, st>>>(a.C, gd, w, b.brick_tot, b.cell_voff, b.T, (uint32_t)nt, b.fix,
-                                            b.fix_cap));
+  if ((e = ensure_entries(b, b.n_cells)) != cudaSuccess) return e;
+  GM_LAUNCH(kc, "k_mc_vertices", st,
+            k_mc_vertices<<<nb, kMcThreads, 0, st>>>(gd, w, b.brick_tot, b.brick_mask, b.cells, b.entries, b.V,
+                                                     a.bbox_min[0], a.bbox_min[1], a.bbox_min[2], cs, a.isovalue));
+  if (b.n_cells > 0)
+    GM_LAUNCH(kc, "k_mc_triangles", st,
+              k_mc_triangles<<<gs_blocks(8 * b.n_cells, kMcThreads, a.num_sms), kMcThreads, 0, st>>>(
+                  gd, w, b.cells, b.entries, (uint32_t)b.n_cells, b.T, (uint32_t)nt, b.fix, b.fix_cap));
   GM_LAUNCH(kc, "k_mc_fix91", st, k_mc_fix91<<<1, 256, 0, st>>>(b.fix, b.fix_cap, b.T));
   if (a.geometry_done) cudaEventRecord(a.geometry_done, st);
   if (nv == 0 || nt == 0) return cudaGetLastError();
