@@ -1662,36 +1662,66 @@ __device__ __forceinline__ uint32_t xrange_mask(int x0, int lo, int hi) {
 __device__ __forceinline__ uint32_t next_cells(uint32_t w, uint32_t after) { return (w >> 8) | (after << 24); }
 __device__ __forceinline__ uint32_t prev_cells(uint32_t w, uint32_t before) { return (w << 8) | before; }
 
+// Blocks of the kernels that walk along z over threads of 16 cells: as many
+// threads along x as the rows have (a power of 2, at most 32), the others
+// along y, `halo` rows of them beside the outputs.  Walks of 16 cells re-read
+// least; shorter ones, down to 2, where the grid gives fewer than 512 blocks
+// (each step waits for its loads).  Tags, selection and contour with 32
+// threads along x and 16 cells against this: 22, 19 and 14 -> 8, 8 and 7 us
+// at 128^3 (walks of 2; 10, 8 and 8 with 4), 53, 49 and 29 -> 35, 25 and 21
+// at 512^3 (walks of 4; 37, 29 and 21 with 2), and at 1024^3 (walks of 16)
+// 166, 137 and 92 (246, 192 and 115 with 2).
+constexpr int kWalkThreads = 320, kWalkBlocks = 512;
+__device__ __forceinline__ bool walk_meets(const CBox& roi, int bx, int out, int z0, int z1) {
+  const int x0 = 16 * (int)blockIdx.x * bx, y0 = (int)blockIdx.y * out;
+  return cbox_meets(roi, x0, x0 + 16 * bx - 1, y0, y0 + out - 1, z0, z1 - 1);
+}
+struct ZWalk {
+  dim3 blocks, threads;
+  int zs;
+};
+static ZWalk z_walk(Dims g, int halo) {
+  int bx = 1;
+  while (16 * bx < g.x && bx < 32) bx *= 2;
+  const int by = kWalkThreads / bx, out = by - halo;
+  ZWalk w;
+  w.threads = dim3(bx, by);
+  const int plane = ((g.x / 16 + bx - 1) / bx) * ((g.y + out - 1) / out);
+  for (w.zs = 16; w.zs > 2 && plane * ((g.z + w.zs - 1) / w.zs) < kWalkBlocks; w.zs /= 2) {}
+  w.blocks = dim3((g.x / 16 + bx - 1) / bx, (g.y + out - 1) / out, (g.z + w.zs - 1) / w.zs);
+  return w;
+}
+
 // Contour of the dilation: fine voxels outside D that are 6-adjacent to D.
 // GM_REF: only for cells in [1, res-2]^3 whose byte is not 0xff
 // (TagVoxelsContourByErosion, Grid.cu:1230-1327); GM_EXACT: whole grid.
-// A block of 32 x 10 threads walks kConZ cells along z, each thread
-// keeping its row of D at z - 1, z, z + 1 in registers; the rows y - 1 and
-// y + 1 come from the neighbouring warps through shared memory (warps 0 and
-// 9 load the halo rows only) and the bytes before and after a thread's 16
-// cells from its neighbouring lanes, so each row of D is read once.
-constexpr int kConZ = 16;
-__global__ void __launch_bounds__(320) k_contour_z(const uint8_t* __restrict__ D, uint8_t* __restrict__ S, Dims g,
-                                                   int exact, CBox roi) {
-  __shared__ uint4 rows_s[10][32];
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  const int x16 = 16 * (blockIdx.x * 32 + tx);
-  const int y = (int)blockIdx.y * 8 - 1 + ty;
-  const int z0 = (int)blockIdx.z * kConZ, z1 = min(z0 + kConZ, g.z);
+// A block walks along z (z_walk), each thread keeping its row of D at z - 1,
+// z, z + 1 in registers; the rows y - 1 and y + 1 come from the block's
+// other threads through shared memory (its first and last rows are halo
+// only) and the bytes before and after a thread's 16 cells from its
+// neighbouring lanes, so each row of D is read once.
+__global__ void __launch_bounds__(kWalkThreads) k_contour_z(const uint8_t* __restrict__ D, uint8_t* __restrict__ S,
+                                                            Dims g, int zs, int exact, CBox roi) {
+  __shared__ uint4 rows_s[kWalkThreads];
+  const int bx = blockDim.x, tx = threadIdx.x, ty = threadIdx.y, me = ty * bx + tx;
+  const int x16 = 16 * (blockIdx.x * bx + tx);
+  const int y = (int)blockIdx.y * (blockDim.y - 2) - 1 + ty;
+  const int z0 = (int)blockIdx.z * zs, z1 = min(z0 + zs, g.z);
+  if (!walk_meets(roi, bx, (int)blockDim.y - 2, z0, z1)) return;
   const bool xok = x16 < g.x, yok = y >= 0 && y < g.y;
   const uint4 z4 = make_uint4(0u, 0u, 0u, 0u);
   auto row = [&](int zz) { return xok && yok && zz >= 0 && zz < g.z ? ld16(D, x16, y, zz, g) : z4; };
   uint4 zm = row(z0 - 1), v = row(z0);
   for (int z = z0; z < z1; z++) {
     const uint4 zp = row(z + 1);
-    rows_s[ty][tx] = v;
+    rows_s[me] = v;
     __syncthreads();
-    uint32_t before = __shfl_up_sync(0xffffffffu, v.w >> 24, 1);
-    uint32_t after = __shfl_down_sync(0xffffffffu, v.x & 0xffu, 1);
-    if (ty >= 1 && ty <= 8 && xok && yok && cbox_meets(roi, x16, x16 + 15, y, y, z, z)) {
+    uint32_t before = __shfl_up_sync(0xffffffffu, v.w >> 24, 1, bx);
+    uint32_t after = __shfl_down_sync(0xffffffffu, v.x & 0xffu, 1, bx);
+    if (ty >= 1 && ty < (int)blockDim.y - 1 && xok && yok && cbox_meets(roi, x16, x16 + 15, y, y, z, z)) {
       if (tx == 0) before = x16 > 0 ? D[cidx(x16 - 1, y, z, g)] : 0u;
-      if (tx == 31 || x16 + 16 >= g.x) after = x16 + 16 < g.x ? D[cidx(x16 + 16, y, z, g)] : 0u;
-      const uint4 ym = rows_s[ty - 1][tx], yp = rows_s[ty + 1][tx];
+      if (tx == bx - 1 || x16 + 16 >= g.x) after = x16 + 16 < g.x ? D[cidx(x16 + 16, y, z, g)] : 0u;
+      const uint4 ym = rows_s[me - bx], yp = rows_s[me + bx];
       const bool yz_in = y >= 1 && z >= 1 && y <= g.y - 2 && z <= g.z - 2;
       uint32_t o[4];
 #pragma unroll
@@ -1757,18 +1787,19 @@ __device__ __forceinline__ void base_dil_row(const uint8_t* X, const uint8_t* Df
   for (int j = 0; j < 4; j++) fr[j] = next_cells(f[j], j < 3 ? f[j + 1] & 0xffu : fa);
 }
 
-// The select kernel computes each base-pass row once: a block of 32 x 9
-// threads walks kSelZ cells along z, each thread keeping its row's flags at
-// z and z + 1 in registers; the row y + 1 comes from the next warp through
-// shared memory (warp 8 computes that halo row only).
-constexpr int kSelZ = 16;
-__global__ void __launch_bounds__(288) k_dil_select_z(const uint8_t* __restrict__ X, const uint8_t* __restrict__ Df,
-                                                      uint8_t* __restrict__ D, Dims g, DataRes dr, CBox roi) {
-  __shared__ uint4 flags_s[9][32][4];  // per thread: f, fr at z; f, fr at z + 1
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  const int x16 = 16 * (blockIdx.x * 32 + tx);
-  const int y = (int)blockIdx.y * 8 + ty;
-  const int z0 = (int)blockIdx.z * kSelZ, z1 = min(z0 + kSelZ, g.z);
+// The select kernel computes each base-pass row once: a block walks along z,
+// each thread keeping its row's flags at z and z + 1 in registers; the row
+// y + 1 comes from the block's next row of threads through shared memory (its
+// last row is that halo only).
+__global__ void __launch_bounds__(kWalkThreads) k_dil_select_z(const uint8_t* __restrict__ X,
+                                                               const uint8_t* __restrict__ Df, uint8_t* __restrict__ D,
+                                                               Dims g, int zs, DataRes dr, CBox roi) {
+  __shared__ uint4 flags_s[4][kWalkThreads];  // per thread: f, fr at z; f, fr at z + 1
+  const int bx = blockDim.x, ty = threadIdx.y, me = ty * bx + threadIdx.x;
+  const int x16 = 16 * (blockIdx.x * bx + threadIdx.x);
+  const int y = (int)blockIdx.y * (blockDim.y - 1) + ty;
+  const int z0 = (int)blockIdx.z * zs, z1 = min(z0 + zs, g.z);
+  if (!walk_meets(roi, bx, (int)blockDim.y - 1, z0, z1)) return;
   const bool xok = x16 < g.x;
   auto row = [&](int zz, uint32_t d0[4], uint32_t f[4], uint32_t fr[4], uint32_t dfw[4]) {
     if (xok) {
@@ -1783,14 +1814,14 @@ __global__ void __launch_bounds__(288) k_dil_select_z(const uint8_t* __restrict_
   for (int z = z0; z < z1; z++) {
     uint32_t d0n[4], fn[4], frn[4], dfn[4];
     row(z + 1, d0n, fn, frn, dfn);
-    flags_s[ty][tx][0] = make_uint4(fc[0], fc[1], fc[2], fc[3]);
-    flags_s[ty][tx][1] = make_uint4(frc[0], frc[1], frc[2], frc[3]);
-    flags_s[ty][tx][2] = make_uint4(fn[0], fn[1], fn[2], fn[3]);
-    flags_s[ty][tx][3] = make_uint4(frn[0], frn[1], frn[2], frn[3]);
+    flags_s[0][me] = make_uint4(fc[0], fc[1], fc[2], fc[3]);
+    flags_s[1][me] = make_uint4(frc[0], frc[1], frc[2], frc[3]);
+    flags_s[2][me] = make_uint4(fn[0], fn[1], fn[2], fn[3]);
+    flags_s[3][me] = make_uint4(frn[0], frn[1], frn[2], frn[3]);
     __syncthreads();
-    if (ty < 8 && xok && y < g.y && cbox_meets(roi, x16, x16 + 15, y, y, z, z)) {
-      const uint4 f1 = flags_s[ty + 1][tx][0], fr1 = flags_s[ty + 1][tx][1];
-      const uint4 f2 = flags_s[ty + 1][tx][2], fr2 = flags_s[ty + 1][tx][3];
+    if (ty < (int)blockDim.y - 1 && xok && y < g.y && cbox_meets(roi, x16, x16 + 15, y, y, z, z)) {
+      const uint4 f1 = flags_s[0][me + bx], fr1 = flags_s[1][me + bx];
+      const uint4 f2 = flags_s[2][me + bx], fr2 = flags_s[3][me + bx];
       // the forward 2x2x2 block mixes full and non-full bytes (cells <= dims - 2)
       const bool yz_ok = y <= g.y - 2 && z <= g.z - 2;
       uint32_t o[4];
@@ -1895,22 +1926,22 @@ static dim3 grid16(Dims g) { return dim3((g.x / 16 + 31) / 32, (g.y + 7) / 8, g.
 // cell) into T and marks the 8^3-cell blocks holding a tagged cell in tmap
 // (zeroed by the caller); once Ef is known on those blocks, k_ero_fix16
 // writes 0xff & ~Ef on the tagged cells.  The bytes equal k_ero_select16's.
-// The tag kernel computes each base-erosion row once: a block of 32 x 10
-// threads walks kTagZ cells along z, each thread keeping its row's C0 at
-// z - 1, z, z + 1 in registers; the rows y - 1 and y + 1 at z come from
-// the neighbouring warps through shared memory (warps 0 and 9 compute the
-// halo rows only), and the bytes before and after a thread's 16 cells from
-// its neighbouring lanes.
-constexpr int kTagZ = 16;
-__global__ void __launch_bounds__(320) k_ero_tag_z(const uint8_t* __restrict__ X, const uint8_t* __restrict__ D,
-                                                   const uint8_t* __restrict__ Eb, uint8_t* __restrict__ C,
-                                                   uint8_t* __restrict__ T, uint8_t* __restrict__ tmap, int mdx,
-                                                   int mdy, Dims g, DataRes dr, CBox roi) {
-  __shared__ uint4 rows_s[10][32];
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  const int x16 = 16 * (blockIdx.x * 32 + tx);
-  const int y = (int)blockIdx.y * 8 - 1 + ty;
-  const int z0 = (int)blockIdx.z * kTagZ, z1 = min(z0 + kTagZ, g.z);
+// The tag kernel computes each base-erosion row once: a block walks along z,
+// each thread keeping its row's C0 at z - 1, z, z + 1 in registers; the rows
+// y - 1 and y + 1 at z come from the block's other threads through shared
+// memory (its first and last rows are halo only), and the bytes before and
+// after a thread's 16 cells from its neighbouring lanes.
+__global__ void __launch_bounds__(kWalkThreads) k_ero_tag_z(const uint8_t* __restrict__ X,
+                                                            const uint8_t* __restrict__ D,
+                                                            const uint8_t* __restrict__ Eb, uint8_t* __restrict__ C,
+                                                            uint8_t* __restrict__ T, uint8_t* __restrict__ tmap,
+                                                            int mdx, int mdy, Dims g, int zs, DataRes dr, CBox roi) {
+  __shared__ uint4 rows_s[kWalkThreads];
+  const int bx = blockDim.x, tx = threadIdx.x, ty = threadIdx.y, me = ty * bx + tx;
+  const int x16 = 16 * (blockIdx.x * bx + tx);
+  const int y = (int)blockIdx.y * (blockDim.y - 2) - 1 + ty;
+  const int z0 = (int)blockIdx.z * zs, z1 = min(z0 + zs, g.z);
+  if (!walk_meets(roi, bx, (int)blockDim.y - 2, z0, z1)) return;
   const bool xok = x16 < g.x, yok = y >= 0 && y < g.y;
   auto row = [&](int zz, uint32_t c[4]) {
     if (xok && yok && zz >= 0 && zz < g.z) {
@@ -1925,13 +1956,13 @@ __global__ void __launch_bounds__(320) k_ero_tag_z(const uint8_t* __restrict__ X
   row(z0, cc);
   for (int z = z0; z < z1; z++) {
     row(z + 1, cn);
-    rows_s[ty][tx] = make_uint4(cc[0], cc[1], cc[2], cc[3]);
+    rows_s[me] = make_uint4(cc[0], cc[1], cc[2], cc[3]);
     __syncthreads();
     // C0 of the cells x16 - 1 and x16 + 16 (the neighbouring lanes' rows;
     // at the block's x edges, from the grid)
-    uint32_t before = __shfl_up_sync(0xffffffffu, cc[3] >> 24, 1);
-    uint32_t after = __shfl_down_sync(0xffffffffu, cc[0] & 0xffu, 1);
-    const bool out = ty >= 1 && ty <= 8 && xok && yok && cbox_meets(roi, x16, x16 + 15, y, y, z, z);
+    uint32_t before = __shfl_up_sync(0xffffffffu, cc[3] >> 24, 1, bx);
+    uint32_t after = __shfl_down_sync(0xffffffffu, cc[0] & 0xffu, 1, bx);
+    const bool out = ty >= 1 && ty < (int)blockDim.y - 1 && xok && yok && cbox_meets(roi, x16, x16 + 15, y, y, z, z);
     if (out) {
       const bool iyz = y < dr.v[1] && z < dr.v[2];
       if (tx == 0)
@@ -1940,15 +1971,15 @@ __global__ void __launch_bounds__(320) k_ero_tag_z(const uint8_t* __restrict__ X
         const int64_t c = cidx(x16 - 1, y, z, g);
         before = c0_of(X[c], D[c], Eb[c], iyz && x16 - 1 < dr.v[0]);
       }
-      if (tx == 31 || x16 + 16 >= g.x) after = 0u;
-      if (tx == 31 && x16 + 16 < g.x) {
+      if (tx == bx - 1 || x16 + 16 >= g.x) after = 0u;
+      if (tx == bx - 1 && x16 + 16 < g.x) {
         const int64_t c = cidx(x16 + 16, y, z, g);
         after = c0_of(X[c], D[c], Eb[c], iyz && x16 + 16 < dr.v[0]);
       }
       const bool interior_yz = y >= 1 && z >= 1 && y <= g.y - 2 && z <= g.z - 2;
       uint32_t tag[4] = {0u, 0u, 0u, 0u};
       if (interior_yz) {
-        const uint4 ym = rows_s[ty - 1][tx], yp = rows_s[ty + 1][tx];
+        const uint4 ym = rows_s[me - bx], yp = rows_s[me + bx];
 #pragma unroll
         for (int j = 0; j < 4; j++) {
           const uint32_t diff = __vcmpne4(cc[j], w_of(ym, j)) | __vcmpne4(cc[j], w_of(yp, j)) |
@@ -2236,9 +2267,9 @@ cudaError_t launch_close(const CloseArgs& a, cudaStream_t st, KernelCounter* kc)
       }
     }
     if (!exact && here()) {
+      const ZWalk w = z_walk(g, 1);
       GM_LAUNCH(kc, "k_dil_select", st,
-                k_dil_select_z<<<dim3((g.x / 16 + 31) / 32, (g.y + 7) / 8, (g.z + kSelZ - 1) / kSelZ), dim3(32, 9), 0,
-                                 st>>>(a.X, Df, D, g, dr, R_D));
+                k_dil_select_z<<<w.blocks, w.threads, 0, st>>>(a.X, Df, D, g, w.zs, dr, R_D));
     }
   } else {
     at += 2;  // the dilation's two passes
@@ -2250,9 +2281,9 @@ cudaError_t launch_close(const CloseArgs& a, cudaStream_t st, KernelCounter* kc)
   }
   // ---- contour ----
   if (here()) {
+    const ZWalk w = z_walk(g, 2);
     GM_LAUNCH(kc, "k_contour", st,
-            k_contour_z<<<dim3((g.x / 16 + 31) / 32, (g.y + 7) / 8, (g.z + kConZ - 1) / kConZ), dim3(32, 10), 0, st>>>(
-                D, S, g, exact ? 1 : 0, R_S));
+              k_contour_z<<<w.blocks, w.threads, 0, st>>>(D, S, g, w.zs, exact ? 1 : 0, R_S));
     // (S holds the refinement tags after the erosion's x pass in GM_REF)
     if (a.S_out) cudaMemcpyAsync(a.S_out, S, cells, cudaMemcpyDeviceToDevice, st);
   }
@@ -2287,9 +2318,9 @@ cudaError_t launch_close(const CloseArgs& a, cudaStream_t st, KernelCounter* kc)
         // blocks of tagged cells (ero y within the z window of them)
         if (here()) {
           cudaMemsetAsync(tmap, 0, (size_t)mdx * mdy * mdz, st);
+          const ZWalk w = z_walk(g, 2);
           GM_LAUNCH(kc, "k_ero_tag", st,
-                    k_ero_tag_z<<<dim3((g.x / 16 + 31) / 32, (g.y + 7) / 8, (g.z + kTagZ - 1) / kTagZ), dim3(32, 10), 0,
-                                  st>>>(a.X, D, Eb, a.C_out, S, tmap, mdx, mdy, g, dr, F));
+                    k_ero_tag_z<<<w.blocks, w.threads, 0, st>>>(a.X, D, Eb, a.C_out, S, tmap, mdx, mdy, g, w.zs, dr, F));
         }
         ok &= dpx_step<KERN_CEN2, uint16_t, 0>(a, at, buf16a, buf16b, nullptr, Nx, Ny, Nz, 1, 0, ehalo, K, RNONE, 0, rx,
                                                ry, st, kc, "k_pass_ero_y", nullptr, 0,
@@ -2416,9 +2447,9 @@ cudaError_t launch_close_zpass(const CloseArgs& a, int z0, int z1, int r_bound, 
 
 cudaError_t launch_contour(const uint8_t* D, uint8_t* S, int res, int exact, cudaStream_t st, KernelCounter* kc) {
   const Dims g{res, res, res};
+  const ZWalk w = z_walk(g, 2);
   GM_LAUNCH(kc, "k_contour", st,
-            k_contour_z<<<dim3((g.x / 16 + 31) / 32, (g.y + 7) / 8, (g.z + kConZ - 1) / kConZ), dim3(32, 10), 0, st>>>(
-                D, S, g, exact, CBox{{0, 0, 0}, {res, res, res}}));
+            k_contour_z<<<w.blocks, w.threads, 0, st>>>(D, S, g, w.zs, exact, CBox{{0, 0, 0}, {res, res, res}}));
   return cudaGetLastError();
 }
 
