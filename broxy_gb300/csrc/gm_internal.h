@@ -40,9 +40,11 @@ struct KernelCounter {
 cudaError_t ensure_dynamic_smem(const void* kernel, size_t bytes);
 
 // The error bits kernels of this library recorded on the current device
-// (kernels with a bounded wait record one; none waits at present), cleared
+// (kernels with a bounded wait record one), cleared
 // when `clear`.
 cudaError_t kernel_error_flags(unsigned int* flags, bool clear);
+// Their device word, for the kernels of other files.
+unsigned int* kernel_error_word();
 
 // JSON {"name": {"launches": n, "ms": t}, ...} of the counter's totals;
 // returns the bytes needed (with the terminating zero), copies when cap allows

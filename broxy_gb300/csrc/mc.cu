@@ -600,8 +600,8 @@ constexpr int kAdjMax = 20;
 constexpr int kAdjRow = 8;
 
 // counters after the vertices' in `cursor`: corners of vertex 0 collected,
-// records placed
-enum { kCntRow0 = 0, kCntRecords = 1, kCntWords = 4 };
+// records placed, blocks that finished an iteration
+enum { kCntRow0 = 0, kCntRecords = 1, kCntArrived = 2, kCntWords = 4 };
 
 __global__ void k_adj_slots(const uint32_t* __restrict__ T, int64_t nt, uint32_t* __restrict__ cursor,
                             uint32_t* __restrict__ adj, uint32_t* __restrict__ adj_more) {
@@ -960,6 +960,91 @@ __global__ void k_bilateral(const float4* __restrict__ Nin, const uint2* __restr
     bilateral_vertex(Nin, rec, roff, v, sn2, zero_isolated, Nout, N3);
 }
 
+// All iterations in one cooperative launch, for meshes whose vertices all fit
+// on the chip as threads: a thread keeps its vertex' first kResGathers records
+// in shared memory, and an iteration is one round of gathers (97 % of the
+// vertices have no more), the same sum in the same order, a store and a
+// barrier over the grid.  A launch per iteration took 7.5 us at 97k vertices,
+// most of it launch, ramp and dependent loads; this takes 4.4, half of it the
+// barrier's round trips (as much with 379 blocks in place of one an SM, and
+// with gathers past L1).
+//
+// The barrier counts arrivals and never resets within a launch (the caller
+// zeroes the counter before it).  The acquire of the count and the block
+// barrier after it order the other blocks' normals before the plain loads of
+// the next iteration.  The blocks are resident together, so the wait ends, and
+// it gives up after kResPolls polls all the same (an error bit).
+constexpr int kResGathers = 8;
+constexpr int kResThreads = 1024;  // at most; one block per SM, so that few arrive
+constexpr uint32_t kResPolls = 1u << 24;
+
+__global__ void __launch_bounds__(kResThreads) k_bilateral_resident(float4* Na, float4* Nb,
+                                                                    const uint2* __restrict__ rec,
+                                                                    const uint32_t* __restrict__ roff, uint32_t nv,
+                                                                    int iters, int zero_isolated, uint32_t* arrived,
+                                                                    float* __restrict__ N3, unsigned int* errors) {
+  extern __shared__ uint32_t mine_s[];  // [2 kResGathers][threads]: the first records' neighbours, then terms
+  const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x, pitch = blockDim.x;
+  uint32_t* mine = mine_s + threadIdx.x;
+  uint32_t n = 0, r0 = 0;
+  float4 na = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (v < nv) {
+    const uint32_t at = roff_at(v);
+    r0 = roff[at], n = roff[at + 1] - r0;
+    na = Na[v];
+    for (uint32_t k = 0; k < kResGathers && k < n; k++) {
+      const uint2 e = rec[r0 + k];
+      mine[k * pitch] = e.x;
+      mine[(kResGathers + k) * pitch] = e.y;
+    }
+  }
+  for (int it = 0; it < iters; it++) {
+    const float sn = it < 2 ? 1e10f : 0.2f, sn2 = sn * sn;  // GMorpho.cu:6959-6969
+    const float4* Nin = (it & 1) ? Nb : Na;
+    float4* Nout = (it & 1) ? Na : Nb;
+    if (v < nv) {
+      float3 nn = make_float3(0.f, 0.f, 0.f);
+      if (!(zero_isolated && n == 0)) {
+        float3 acc = make_float3(0.f, 0.f, 0.f);
+        float4 nb[kResGathers];
+#pragma unroll
+        for (int k = 0; k < kResGathers; k++)
+          if (k < n) nb[k] = Nin[mine[k * pitch]];
+#pragma unroll
+        for (int k = 0; k < kResGathers; k++)
+          if (k < n) bilateral_add(acc, make_uint2(0u, mine[(kResGathers + k) * pitch]), nb[k], na, sn2);
+        for (uint32_t i = kResGathers; i < n; i++) {
+          const uint2 e = rec[r0 + i];
+          bilateral_add(acc, e, Nin[e.x], na, sn2);
+        }
+        nn = normalize3(acc);
+      }
+      na = make_float4(nn.x, nn.y, nn.z, 0.f);
+      if (it == iters - 1) {
+        float* o = N3 + 3 * (size_t)v;
+        o[0] = nn.x; o[1] = nn.y; o[2] = nn.z;
+      } else {
+        __stcg(Nout + v, na);
+      }
+    }
+    if (it == iters - 1) return;
+    __syncthreads();
+    int ok = 1;
+    if (threadIdx.x == 0) {
+      const uint32_t want = (uint32_t)(it + 1) * gridDim.x;
+      __threadfence();  // the block's normals before its arrival
+      atomicAdd(arrived, 1u);
+      uint32_t seen, polls = 0;
+      do {
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(arrived) : "memory");
+        ok = ++polls < kResPolls;
+      } while (seen < want && ok);
+      if (!ok) atomicOr(errors, 1u);
+    }
+    if (!__syncthreads_and(ok)) return;
+  }
+}
+
 // The same iteration over the vertices of several meshes at once (one
 // launch per iteration for a batch): vertex g of the concatenation belongs
 // to the mesh m with start[m] <= g < start[m + 1].
@@ -1234,6 +1319,24 @@ cudaError_t mesh_emit(const MeshArgs& a, MeshBuffers& b, int64_t nv, int64_t nt,
   if (a.defer_filter) return cudaGetLastError();
   float4* nin = b.N4a;
   float4* nout = b.N4b;
+  const int64_t share = nv / (sms > 0 ? sms : 152) / 32 * 32 + 32;  // vertices of an SM, whole warps
+  const int res_threads = (int)(share < 128 ? 128 : share);
+  if (iters > 1 && res_threads <= kResThreads) {
+    uint32_t nv32 = (uint32_t)nv, *arrived = counters + kCntArrived;
+    unsigned int* errors = kernel_error_word();
+    void* args[] = {&b.N4a, &b.N4b, &b.rec, &b.roff, &nv32, const_cast<int*>(&iters), const_cast<int*>(&zi),
+                    &arrived, &b.N, &errors};
+    const size_t res_smem = 2 * kResGathers * sizeof(uint32_t) * (size_t)res_threads;
+    cudaError_t le = ensure_dynamic_smem(reinterpret_cast<const void*>(k_bilateral_resident), res_smem);
+    if (le != cudaSuccess) return le;
+    GM_LAUNCH(kc, "k_bilateral", st,
+              le = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_bilateral_resident),
+                                               dim3((unsigned)((nv + res_threads - 1) / res_threads)),
+                                               dim3((unsigned)res_threads), args, res_smem, st));
+    if (le == cudaSuccess) return cudaGetLastError();
+    if (le != cudaErrorCooperativeLaunchTooLarge) return le;
+    cudaGetLastError();  // fewer SMs than the device has: an iteration per launch
+  }
   const int bil_blocks = wave_blocks(reinterpret_cast<const void*>(k_bilateral), nv, sms);
   for (int it = 0; it < iters; it++) {
     const float sn = it < 2 ? 1e10f : 0.2f;  // GMorpho.cu:6959-6969

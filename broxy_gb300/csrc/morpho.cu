@@ -34,7 +34,8 @@
 namespace gm {
 
 // Error bits that kernels with a bounded wait record instead of trapping
-// (none waits at present); read and cleared by kernel_error_flags().
+// (bit 0: the grid barrier of the resident normal filter gave up); read and
+// cleared by kernel_error_flags().
 __device__ unsigned int g_kernel_errors = 0;
 
 // A radius field read in place: element (x, y, z) at p[x + y sy + z sz]
@@ -1471,6 +1472,11 @@ static bool dpx_step(const CloseArgs& a, int& at, const TIn* in, uint16_t* out16
                                                         uniform_r, rx, ry, rmap, rext, need);
   at++;
   return ok;
+}
+
+unsigned int* kernel_error_word() {
+  void* p = nullptr;
+  return cudaGetSymbolAddress(&p, g_kernel_errors) == cudaSuccess ? static_cast<unsigned int*>(p) : nullptr;
 }
 
 cudaError_t kernel_error_flags(unsigned int* flags, bool clear) {

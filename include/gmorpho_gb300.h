@@ -92,8 +92,9 @@ const char* gm_ctx_last_error(const gm_ctx* ctx);
 long long gm_ctx_kernel_launches(const gm_ctx* ctx);
 /* Error bits that this library's kernels recorded on the current device
  * instead of trapping: bit 0 = a bounded wait of a kernel ran out (the
- * results of that call are not trustworthy; no kernel waits at present, so
- * none sets it).  Waits for the device's work; clears the bits when `clear`.
+ * results of that call are not trustworthy; the grid barrier of the normal
+ * filter on small meshes is the one that waits).  Waits for the device's
+ * work; clears the bits when `clear`.
  * No counterpart in the reference (which checks cudaGetLastError only,
  * GMorpho/GMorpho.cu:50-56). */
 gm_status gm_kernel_error_flags(uint32_t* flags, int32_t clear);

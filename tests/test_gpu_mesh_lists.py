@@ -65,3 +65,16 @@ def test_border(gm_ctx, cut):
     z, y, x = np.meshgrid(*[np.arange(32)] * 3, indexing="ij")
     occ = (x - (2.5 - 2 * cut)) ** 2 + (y - 16) ** 2 + (z - 16) ** 2 < 36
     _check(gm_ctx, occ, 4)
+
+
+@pytest.mark.parametrize("blocks", [6475, 6490])
+@pytest.mark.parametrize("iters", [1, 3])
+def test_filter_around_one_vertex_a_thread(gm_ctx, blocks, iters):
+    """Solid 2x2x2 blocks, 24 vertices each: 155400 and 155760 vertices, about
+    as many as the chip holds threads of the resident filter (155648)."""
+    occ = np.zeros((128, 128, 128), bool)
+    at = np.stack(np.meshgrid(*[np.arange(4, 124, 5)] * 3, indexing="ij"), -1).reshape(-1, 3)[:blocks]
+    for z, y, x in at:
+        occ[z:z + 2, y:y + 2, x:x + 2] = True
+    assert _check(gm_ctx, occ, iters)[0] == 24 * blocks
+    assert api.kernel_error_flags() == 0
