@@ -269,7 +269,7 @@ struct MeshBuffers {
                             // neighbour), packed in chunks of 256 vertices
   uint32_t* roff = nullptr; // v_cap + v_cap / 256 + 4: their offsets, 257 a chunk after vertex 0's two
   uint32_t* T = nullptr;    // 3 * t_cap
-  uint32_t* row0 = nullptr; // 3 * t_cap: corners of vertex 0 where they are many
+  uint32_t* row0 = nullptr; // 3 * t_cap: corners of vertex 0
   uint32_t* adj = nullptr;  // 20 * v_cap: corner rows (8 slots a vertex, then 12 more each)
   uint32_t* cursor = nullptr;  // v_cap corner counts, then the mesh's counters
   int64_t v_cap = 0, t_cap = 0;
@@ -281,7 +281,7 @@ struct MeshBuffers {
   int64_t entries_cap = 0, n_cells = 0;
   uint32_t* fix = nullptr;        // case-91 fix list: 1 + 4 * fix_cap
   int64_t cells_cap = 0, bricks_cap = 0;
-  int fix_cap = 0;
+  int fix_cap = 0, n_fix = 0;
 };
 
 // Phase 1: counts (host-synchronous: returns the vertex/triangle totals).

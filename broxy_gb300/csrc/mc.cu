@@ -599,27 +599,20 @@ __global__ void k_mc_fix91(const uint32_t* __restrict__ fix, int fix_cap, uint32
 constexpr int kAdjMax = 20;
 constexpr int kAdjRow = 8;
 
-// counters after the vertices' in `cursor`: corners of vertex 0 collected,
-// records placed, blocks that finished an iteration
-enum { kCntRow0 = 0, kCntRecords = 1, kCntArrived = 2, kCntWords = 4 };
+// counters after the vertices' in `cursor`: records placed, blocks that
+// finished an iteration
+enum { kCntRecords = 0, kCntArrived = 1, kCntWords = 4 };
 
 __global__ void k_adj_slots(const uint32_t* __restrict__ T, int64_t nt, uint32_t* __restrict__ cursor,
-                            uint32_t* __restrict__ adj, uint32_t* __restrict__ adj_more) {
+                            uint32_t* __restrict__ adj, uint32_t* __restrict__ adj_more,
+                            uint32_t* __restrict__ row0) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < 3 * nt; i += (int64_t)gridDim.x * blockDim.x) {
     const uint32_t v = T[i];
     const uint32_t slot = atomicAdd(cursor + v, 1u);
     if (slot < kAdjRow) adj[(size_t)kAdjRow * v + slot] = (uint32_t)i;  // corner id = 3 t + role
     else if (slot < kAdjMax) adj_more[(size_t)(kAdjMax - kAdjRow) * v + slot - kAdjRow] = (uint32_t)i;
+    if (v == 0u) row0[slot] = (uint32_t)i;
   }
-}
-
-// The corners of a vertex 0 that has more than kAdjMax of them (else nothing
-// to do), in any order.
-__global__ void k_row0_collect(const uint32_t* __restrict__ T, int64_t nt, const uint32_t* __restrict__ cursor,
-                               uint32_t* __restrict__ counters, uint32_t* __restrict__ row0) {
-  if (cursor[0] <= kAdjMax) return;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < 3 * nt; i += (int64_t)gridDim.x * blockDim.x)
-    if (T[i] == 0u) row0[atomicAdd(counters + kCntRow0, 1u)] = (uint32_t)i;
 }
 
 __device__ __forceinline__ float3 ld3(const float* p, uint32_t i) {
@@ -697,6 +690,7 @@ __device__ __forceinline__ float3 add3(float3 a, float3 b) {
 // of eight slots a vertex, or slots of 32 vertices interleaved, were 18%
 // slower.)
 constexpr int kRecChunk = 256;
+constexpr int kPool = 4;  // general vertices that a warp takes together (more go one a lane)
 __device__ __forceinline__ uint32_t roff_at(uint32_t v) { return v == 0u ? 0u : v + v / kRecChunk + 2u; }
 
 // pairs (neighbour << 32 | term bits) sorted; merged in place into records
@@ -749,6 +743,69 @@ __device__ __noinline__ float3 finish_general(const float* __restrict__ V, const
   return acc;
 }
 
+// The same by a warp whose lanes hold the corners (all lanes call it; n at
+// most kAdjMax): ranks instead of sorts, so that a vertex costs its three
+// dependent loads and a few hundred instructions, not a chain of them: nearly
+// every chunk has one (0.3 % of a solid's vertices have more than eight
+// corners) and waited for it, 27 -> 18.5 us at 97k vertices, 0.471 -> 0.416 ms
+// at 5.7M.
+__device__ __noinline__ float3 finish_by_warp(const float* __restrict__ V, const uint32_t* __restrict__ T, uint32_t v,
+                                              uint32_t n, const uint32_t* __restrict__ adj,
+                                              const uint32_t* __restrict__ adj_more, bool records_wanted, uint64_t* kv,
+                                              uint32_t* records) {
+  const uint32_t lane = threadIdx.x & 31;
+  const bool has = lane < n;
+  uint32_t key = 0xffffffffu, id[2] = {0xffffffffu, 0xffffffffu}, rank = 0;
+  float3 nn = make_float3(0.f, 0.f, 0.f), acc = nn;
+  if (has) {
+    key = lane < kAdjRow ? adj[(size_t)kAdjRow * v + lane]
+                         : adj_more[(size_t)(kAdjMax - kAdjRow) * v + lane - kAdjRow];
+    adj_corner(V, T, key, nn, id[0], id[1]);
+  }
+  for (uint32_t j = 0; j < n; j++) rank += __shfl_sync(0xffffffffu, key, j) < key;
+  for (uint32_t j = 0; j < n; j++) {
+    const int src = __ffs(__ballot_sync(0xffffffffu, has && rank == j)) - 1;
+    acc = add3(acc, make_float3(__shfl_sync(0xffffffffu, nn.x, src), __shfl_sync(0xffffffffu, nn.y, src),
+                                __shfl_sync(0xffffffffu, nn.z, src)));
+  }
+  *records = 0;
+  if (!records_wanted) return acc;
+  // a neighbour's occurrences have one term, so they differ by their place
+  // (2 lane + h) only: every second one is kept, as a double if it has a next
+  uint32_t less[2] = {0, 0}, run[2] = {0, 0}, all[2] = {0, 0};
+  for (uint32_t j = 0; j < n; j++) {
+    const uint32_t a = __shfl_sync(0xffffffffu, id[0], j), b = __shfl_sync(0xffffffffu, id[1], j);
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      less[h] += (a < id[h]) + (b < id[h]);
+      all[h] += (a == id[h]) + (b == id[h]);
+      run[h] += (a == id[h] && (h == 0 ? j < lane : j <= lane)) + (b == id[h] && j < lane);
+    }
+  }
+  uint32_t lo = 0, hi = 0;
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const uint32_t at = less[h] + run[h];  // its place in (neighbour, occurrence) order
+    if (has && !(run[h] & 1)) (at < 32 ? lo : hi) |= 1u << (at & 31);
+  }
+  lo = __reduce_or_sync(0xffffffffu, lo);
+  hi = __reduce_or_sync(0xffffffffu, hi);
+  const float3 pa = ld3(V, v);
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const uint32_t at = less[h] + run[h];
+    if (has && !(run[h] & 1)) {
+      const uint32_t place = __popc(lo & (at < 32 ? (1u << at) - 1u : 0xffffffffu)) +
+                             (at < 32 ? 0 : __popc(hi & ((1u << (at - 32)) - 1u)));
+      kv[place] = ((uint64_t)id[h] << 32) | __float_as_uint(dist2(pa, ld3(V, id[h]))) |
+                  (run[h] + 1 < all[h] ? 0x80000000u : 0u);
+    }
+  }
+  *records = __popc(lo) + __popc(hi);
+  __syncwarp();
+  return acc;
+}
+
 // The per-vertex steps after the corner rows are filled, in one kernel: the
 // row sorted into triangle order; the area-weighted normal summed in that
 // order and normalised (GMorpho.cu:6498-6537); and, when the normals are
@@ -767,6 +824,8 @@ __global__ void __launch_bounds__(kRecChunk, 4) k_adj_finish(const float* __rest
                              int zero_isolated, float4* __restrict__ N4, float* __restrict__ N3,
                              uint2* __restrict__ rec, uint32_t* __restrict__ roff, uint32_t* __restrict__ counters) {
   __shared__ uint32_t base_s;
+  __shared__ uint64_t pool[kRecChunk / 32][kPool][2 * kAdjMax];  // records of a warp's general vertices
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int64_t v = blockIdx.x * (int64_t)kRecChunk + threadIdx.x;
   const uint32_t n = v < nv ? cursor[v] : 0u;
   const bool isolated = n == 0 && (zero_isolated || v >= nv);
@@ -807,7 +866,16 @@ __global__ void __launch_bounds__(kRecChunk, 4) k_adj_finish(const float* __rest
       }
     }
   }
-  if (here && !fan) acc = finish_general(V, T, v, n, adj, adj_more, ld3(V, (uint32_t)v), kv, &records);
+  int slot = -1, used = 0;
+  for (uint32_t todo = __ballot_sync(0xffffffffu, here && !fan); todo && used < kPool; used++) {
+    const int src = __ffs(todo) - 1;
+    todo &= todo - 1;
+    uint32_t count;
+    const float3 sum = finish_by_warp(V, T, (uint32_t)(v - lane + src), __shfl_sync(0xffffffffu, n, src), adj, adj_more,
+                                      rec != nullptr, pool[wid][used], &count);
+    if (lane == src) acc = sum, records = count, slot = used;
+  }
+  if (here && !fan && slot < 0) acc = finish_general(V, T, v, n, adj, adj_more, ld3(V, (uint32_t)v), kv, &records);
   if (rec) {
     uint32_t total;
     const uint32_t pre = block_scan1(records, total);
@@ -822,8 +890,13 @@ __global__ void __launch_bounds__(kRecChunk, 4) k_adj_finish(const float* __rest
 #pragma unroll
       for (int k = 0; k < 8; k++)
         if ((uint32_t)k < records) rec[at + k] = make_uint2(p[k], t[k]);
-    } else {
+    } else if (slot < 0) {
       for (uint32_t i = 0; i < records; i++) rec[at + i] = as_record(kv[i]);
+    }
+    for (int u = 0; u < used; u++) {
+      const int src = __ffs(__ballot_sync(0xffffffffu, slot == u)) - 1;
+      const uint32_t to = __shfl_sync(0xffffffffu, at, src), count = __shfl_sync(0xffffffffu, records, src);
+      for (uint32_t i = lane; i < count; i += 32) rec[to + i] = as_record(pool[wid][u][i]);
     }
   }
   if (v >= nv || !(here || isolated)) return;
@@ -1234,7 +1307,8 @@ cudaError_t mesh_count_launch(const MeshArgs& a, MeshBuffers& b, cudaStream_t st
   {
     const int nchunks = (nb + kBrickChunk - 1) / kBrickChunk;
     if (nchunks > kBrickChunk) return cudaErrorInvalidValue;
-    GM_LAUNCH(kc, "k_brick_sums", st, k_brick_sums<<<nchunks, kBrickChunk, 0, st>>>(b.brick_tot, nb));
+    if (nchunks > 1)  // (one chunk's scan reads no sums)
+      GM_LAUNCH(kc, "k_brick_sums", st, k_brick_sums<<<nchunks, kBrickChunk, 0, st>>>(b.brick_tot, nb));
     GM_LAUNCH(kc, "k_scan_bricks", st, k_scan_bricks<<<nchunks, kBrickChunk, 0, st>>>(b.brick_tot, nb));
   }
   return cudaMemcpyAsync(h_tot4, b.brick_tot + 4 * (size_t)nb, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
@@ -1250,7 +1324,7 @@ cudaError_t mesh_count_finish(MeshBuffers& b, const uint32_t* tot, int64_t* nv, 
   b.n_cells = tot[0];
   *nv = tot[1];
   *nt = tot[2];
-  const int need_fix = (int)tot[3];
+  const int need_fix = b.n_fix = (int)tot[3];
   if (need_fix + 1 > b.fix_cap || b.fix == nullptr) {
     if (b.fix) cudaFree(b.fix);
     b.fix = nullptr;
@@ -1286,7 +1360,7 @@ cudaError_t mesh_emit(const MeshArgs& a, MeshBuffers& b, int64_t nv, int64_t nt,
   if ((e = ensure_vertex_buffers(b, nv)) != cudaSuccess) return e;
   if ((e = ensure_triangle_buffers(b, nt)) != cudaSuccess) return e;
   const float cs = 0.5f * a.cell_size;  // exact: scaling by a power of two
-  cudaMemsetAsync(b.fix, 0, sizeof(uint32_t), st);
+  if (b.n_fix > 0) cudaMemsetAsync(b.fix, 0, sizeof(uint32_t), st);
   if ((e = ensure_entries(b, b.n_cells)) != cudaSuccess) return e;
   GM_LAUNCH(kc, "k_mc_vertices", st,
             k_mc_vertices<<<nb, kMcThreads, 0, st>>>(gd, w, b.brick_tot, b.brick_mask, b.cells, b.entries, b.V,
@@ -1295,7 +1369,7 @@ cudaError_t mesh_emit(const MeshArgs& a, MeshBuffers& b, int64_t nv, int64_t nt,
     GM_LAUNCH(kc, "k_mc_triangles", st,
               k_mc_triangles<<<gs_blocks(8 * b.n_cells, kMcThreads, a.num_sms), kMcThreads, 0, st>>>(
                   gd, w, b.cells, b.entries, (uint32_t)b.n_cells, b.T, (uint32_t)nt, b.fix, b.fix_cap));
-  GM_LAUNCH(kc, "k_mc_fix91", st, k_mc_fix91<<<1, 256, 0, st>>>(b.fix, b.fix_cap, b.T));
+  if (b.n_fix > 0) GM_LAUNCH(kc, "k_mc_fix91", st, k_mc_fix91<<<1, 256, 0, st>>>(b.fix, b.fix_cap, b.T));
   if (a.geometry_done) cudaEventRecord(a.geometry_done, st);
   if (nv == 0 || nt == 0) return cudaGetLastError();
   // normals
@@ -1308,9 +1382,7 @@ cudaError_t mesh_emit(const MeshArgs& a, MeshBuffers& b, int64_t nv, int64_t nt,
   float* n3 = iters == 0 ? b.N : nullptr;
   cudaMemsetAsync(b.cursor, 0, sizeof(uint32_t) * (size_t)(nv + kCntWords), st);
   GM_LAUNCH(kc, "k_adj_slots", st,
-            k_adj_slots<<<gs_blocks(3 * nt, 256, sms), 256, 0, st>>>(b.T, nt, b.cursor, b.adj, adj_more));
-  GM_LAUNCH(kc, "k_row0_collect", st,
-            k_row0_collect<<<gs_blocks(3 * nt, 256, sms), 256, 0, st>>>(b.T, nt, b.cursor, counters, b.row0));
+            k_adj_slots<<<gs_blocks(3 * nt, 256, sms), 256, 0, st>>>(b.T, nt, b.cursor, b.adj, adj_more, b.row0));
   GM_LAUNCH(kc, "k_adj_finish", st,
             k_adj_finish<<<(unsigned)((nv + kRecChunk - 1) / kRecChunk), kRecChunk, 0, st>>>(
                 b.V, b.T, b.cursor, b.adj, adj_more, nv, zi, b.N4a, n3, rec, b.roff, counters));
