@@ -100,11 +100,11 @@ struct TriD {
   double g[3][3];  // vertices in voxels
 };
 
-__device__ __forceinline__ void tri_load(const float* __restrict__ P, const uint32_t* __restrict__ T, int64_t t,
+__device__ __forceinline__ void tri_load(const float* __restrict__ P, const uint32_t* __restrict__ T, uint32_t t,
                                          const VoxParams& vp, TriD& d) {
   for (int j = 0; j < 3; j++)
     for (int a = 0; a < 3; a++)
-      d.g[j][a] = __ddiv_rn(dsub((double)P[3 * (size_t)T[3 * t + j] + a], (double)vp.b[a]), vp.h);
+      d.g[j][a] = __ddiv_rn(dsub((double)P[3 * (size_t)T[3 * (size_t)t + j] + a], (double)vp.b[a]), vp.h);
 }
 
 // (i) volume parity: pixel (x, y) flips the voxel at floor(z) of its centre
@@ -183,8 +183,8 @@ __device__ __forceinline__ uint32_t* zword(uint32_t* g, int N, int x, int y) {
   return g + ((int64_t)x + (int64_t)N * y) * (N >> 5);
 }
 
-// Calls of the float form for what it cannot decide (rare: out of line)
-__device__ __noinline__ void ask_pixel(const float* __restrict__ P, const uint32_t* __restrict__ T, int64_t t, int x,
+// What the float form cannot decide (rare: out of line)
+__device__ __noinline__ void ask_pixel(const float* __restrict__ P, const uint32_t* __restrict__ T, uint32_t t, int x,
                                        int y, const VoxParams& vp) {
   TriD d;
   tri_load(P, T, t, vp, d);
@@ -193,7 +193,7 @@ __device__ __noinline__ void ask_pixel(const float* __restrict__ P, const uint32
   if (x >= x0 && x <= x1 && y >= y0 && y <= y1) pixel_exact(d, x, y, vp);
 }
 
-__device__ __noinline__ void ask_voxels(const float* __restrict__ P, const uint32_t* __restrict__ T, int64_t t, int x,
+__device__ __noinline__ void ask_voxels(const float* __restrict__ P, const uint32_t* __restrict__ T, uint32_t t, int x,
                                         int y, int z0, int z1, const VoxParams& vp) {
   TriD d;
   tri_load(P, T, t, vp, d);
@@ -204,7 +204,37 @@ __device__ __noinline__ void ask_voxels(const float* __restrict__ P, const uint3
     if (voxel_exact(d, x, y, z)) atomicOr(zword(vp.surf, vp.N, x, y) + (z >> 5), 1u << (z & 31));
 }
 
-__device__ __noinline__ bool ask_surface(const float* __restrict__ P, const uint32_t* __restrict__ T, int64_t t,
+// Such tests of a warp's walks, kept for the end, where its lanes make them
+// together: a test takes microseconds at the rate of FP64 here, and the warp
+// waited for each of them: 42 -> 34 us for 82k triangles into 128^3, and
+// 84 where one warp had many.
+constexpr uint32_t kAsks = 32;
+constexpr int kVoxThreads = 64;
+struct Asks {
+  uint32_t n;
+  uint4 q[kAsks];  // triangle, x | y << 16, first and last z; first z -1: the column's pixel
+};
+__device__ __forceinline__ void make_ask(const float* __restrict__ P, const uint32_t* __restrict__ T, uint4 a,
+                                         const VoxParams& vp) {
+  const int x = (int)(a.y & 0xffffu), y = (int)(a.y >> 16);
+  if ((int)a.z < 0) ask_pixel(P, T, a.x, x, y, vp);
+  else ask_voxels(P, T, a.x, x, y, (int)a.z, (int)a.w, vp);
+}
+__device__ __forceinline__ Asks& warp_asks() {
+  __shared__ Asks asks[kVoxThreads / 32];
+  return asks[threadIdx.x >> 5];
+}
+// (KEEP false: at once)
+template <bool KEEP>
+__device__ __forceinline__ void ask(const float* __restrict__ P, const uint32_t* __restrict__ T, uint32_t t, int x,
+                                    int y, int z0, int z1, const VoxParams& vp) {
+  const uint4 a = make_uint4(t, (uint32_t)x | ((uint32_t)y << 16), (uint32_t)z0, (uint32_t)z1);
+  const uint32_t i = KEEP ? atomicAdd(&warp_asks().n, 1u) : kAsks;
+  if (i < kAsks) warp_asks().q[i] = a;
+  else make_ask(P, T, a, vp);
+}
+
+__device__ __noinline__ bool ask_surface(const float* __restrict__ P, const uint32_t* __restrict__ T, uint32_t t,
                                          const VoxParams& vp) {
   TriD d;
   tri_load(P, T, t, vp, d);
@@ -224,8 +254,8 @@ __device__ __noinline__ bool ask_surface(const float* __restrict__ P, const uint
 // vertices' coordinates are computed as a pair of floats (46 bits), so no
 // double arithmetic is left on the common path: FP64 issues at 1/64 of the
 // FP32 rate here and was what bounded the voxelizer (115 ms for 4.0M
-// triangles into 1024^3, 1.94 ms for 82k into 128^3; k_vox_tris: 0.85 and
-// 0.042 ms).
+// triangles into 1024^3, 1.94 ms for 82k into 128^3; k_vox_tris: 0.84 and
+// 0.034 ms).
 struct Slab {
   // z interval at the column coordinate u: [lo - k u, hi - k u], rounding
   // within w; a slab that hardly depends on z (flat) is a test of k u
@@ -285,13 +315,13 @@ enum TriClass { TRI_FLOAT = 0, TRI_EXACT = 1 };
 
 // The float form of a triangle.  TRI_EXACT: outside its range (coordinates
 // of 4096 voxels or more or not finite, a degenerate size).
-__device__ __forceinline__ TriClass tri_setup(const float* __restrict__ P, const uint32_t* __restrict__ T, int64_t t,
+__device__ __forceinline__ TriClass tri_setup(const float* __restrict__ P, const uint32_t* __restrict__ T, uint32_t t,
                                               const VoxParams& vp, TriF& f) {
   float p[3][3], q[3][3], v[3][3], e[3][3];
   bool ok = true;
 #pragma unroll
   for (int j = 0; j < 3; j++) {
-    const float* src = P + 3 * (size_t)T[3 * t + j];
+    const float* src = P + 3 * (size_t)T[3 * (size_t)t + j];
 #pragma unroll
     for (int a = 0; a < 3; a++) {
       // (P - b) / h as a pair of floats: an exact two-float difference times
@@ -388,7 +418,8 @@ __device__ __forceinline__ TriClass tri_setup(const float* __restrict__ P, const
 }
 
 // One column of a triangle: parity pixel and surface voxels
-__device__ __forceinline__ void tri_column(const float* __restrict__ P, const uint32_t* __restrict__ T, int64_t t,
+template <bool KEEP>
+__device__ __forceinline__ void tri_column(const float* __restrict__ P, const uint32_t* __restrict__ T, uint32_t t,
                                            const VoxParams& vp, const TriF& f, int x, int y, ZRange zr, bool zy_in) {
   const int N = vp.N;
   const float X = (float)(x - f.o[0]) + 0.5f, Y = (float)(y - f.o[1]) + 0.5f;
@@ -421,7 +452,7 @@ __device__ __forceinline__ void tri_column(const float* __restrict__ P, const ui
         atomicXor(zword(vp.mark, N, x, y) + (k >> 5), 1u << (k & 31));
       }
     } else {
-      ask_pixel(P, T, t, x, y, vp);
+      ask<KEEP>(P, T, t, x, y, -1, -1, vp);
     }
   }
   // (ii) surface
@@ -445,8 +476,8 @@ __device__ __forceinline__ void tri_column(const float* __restrict__ P, const ui
     atomicOr(col + w, (0xffffffffu >> (31 - (last - z))) << (z & 31));
     z = last + 1;
   }
-  if (d0 > p0) ask_voxels(P, T, t, x, y, p0, min(d0 - 1, p1), vp);
-  if (d0 <= d1 && d1 < p1) ask_voxels(P, T, t, x, y, d1 + 1, p1, vp);
+  if (d0 > p0) ask<KEEP>(P, T, t, x, y, p0, min(d0 - 1, p1), vp);
+  if (d0 <= d1 && d1 < p1) ask<KEEP>(P, T, t, x, y, d1 + 1, p1, vp);
 }
 
 // z interval of the yz slabs of a row of columns; false: no voxel passes
@@ -463,32 +494,38 @@ __device__ __forceinline__ bool tri_row(const TriF& f, int y, ZRange& zr) {
 // One thread per triangle of at most kVoxCols columns; larger ones are
 // listed from the front, those outside the float form's range from the back
 // (counts: [0] large, [1] exact).  Bound by the latency of a warp's longest
-// walk (a triangle of the 1024^3 case has five columns on average, up to a
-// dozen): three blocks an SM (168 registers, no spills to speak of) took
-// 0.85 ms, two blocks 1.00, four (128 registers) 0.95.
+// walk (a triangle of a 4.0M-triangle surface in 1024^3 has five columns on
+// average, up to a dozen): six blocks of 64 an SM (168 registers, no spills
+// to speak of) take 0.84 ms, a third fewer warps 1.00, a third more (128
+// registers) 0.95; blocks of 128 were 3 % slower, seven of 64 32 %.
 constexpr int kVoxCols = 64;
-__global__ void __launch_bounds__(128, 3) k_vox_tris(const float* __restrict__ P, const uint32_t* __restrict__ T,
-                                                  int64_t nf, const __grid_constant__ VoxParams vp,
+__global__ void __launch_bounds__(kVoxThreads, 6) k_vox_tris(const float* __restrict__ P, const uint32_t* __restrict__ T,
+                                                  uint32_t nf, const __grid_constant__ VoxParams vp,
                                                   uint32_t* __restrict__ list, uint32_t* __restrict__ counts) {
-  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (t >= nf) return;
-  TriF f;
-  if (tri_setup(P, T, t, vp, f) == TRI_EXACT) {
-    list[nf - 1 - atomicAdd(counts + 1, 1u)] = (uint32_t)t;
-    return;
+  if ((threadIdx.x & 31) == 0) warp_asks().n = 0;
+  __syncwarp();
+  const uint32_t t = blockIdx.x * kVoxThreads + threadIdx.x;  // (at most kVoxChunk)
+  if (t < nf) {
+    TriF f;
+    if (tri_setup(P, T, t, vp, f) == TRI_EXACT) {
+      list[nf - 1 - atomicAdd(counts + 1, 1u)] = t;
+    } else {
+      const int nx = f.hi[0] - f.lo[0] + 1, ny = f.hi[1] - f.lo[1] + 1;
+      if (nx > 0 && ny > 0 && (nx > kVoxCols || ny > kVoxCols || nx * ny > kVoxCols)) {
+        list[atomicAdd(counts, 1u)] = t;
+      } else if (nx > 0) {
+        for (int y = f.lo[1]; y <= f.hi[1]; y++) {
+          ZRange zr;
+          const bool zy = tri_row(f, y, zr);
+          if (!zy) zr.phi = -1e30f, zr.plo = 1e30f;  // pixels only
+          for (int x = f.lo[0]; x <= f.hi[0]; x++) tri_column<true>(P, T, t, vp, f, x, y, zr, zy);
+        }
+      }
+    }
   }
-  const int nx = f.hi[0] - f.lo[0] + 1, ny = f.hi[1] - f.lo[1] + 1;
-  if (nx <= 0 || ny <= 0) return;
-  if (nx > kVoxCols || ny > kVoxCols || nx * ny > kVoxCols) {
-    list[atomicAdd(counts, 1u)] = (uint32_t)t;
-    return;
-  }
-  for (int y = f.lo[1]; y <= f.hi[1]; y++) {
-    ZRange zr;
-    const bool zy = tri_row(f, y, zr);
-    if (!zy) zr.phi = -1e30f, zr.plo = 1e30f;  // pixels only
-    for (int x = f.lo[0]; x <= f.hi[0]; x++) tri_column(P, T, t, vp, f, x, y, zr, zy);
-  }
+  __syncwarp();
+  const uint32_t lane = threadIdx.x & 31;
+  if (lane < min(warp_asks().n, kAsks)) make_ask(P, T, warp_asks().q[lane], vp);
 }
 
 // One block per listed triangle, its threads over the columns of a large
@@ -499,7 +536,7 @@ __global__ void __launch_bounds__(128) k_vox_listed(const float* __restrict__ P,
                                                     const uint32_t* __restrict__ counts) {
   const uint32_t n = counts[0], m = counts[1];
   for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {
-    const int64_t t = list[i];
+    const uint32_t t = list[i];
     TriF f;
     tri_setup(P, T, t, vp, f);
     const int nx = f.hi[0] - f.lo[0] + 1, ny = f.hi[1] - f.lo[1] + 1;
@@ -508,7 +545,7 @@ __global__ void __launch_bounds__(128) k_vox_listed(const float* __restrict__ P,
       ZRange zr;
       const bool zy = tri_row(f, y, zr);
       if (!zy) zr.phi = -1e30f, zr.plo = 1e30f;
-      tri_column(P, T, t, vp, f, x, y, zr, zy);
+      tri_column<false>(P, T, t, vp, f, x, y, zr, zy);
     }
   }
   for (uint32_t i = blockIdx.x; i < m; i += gridDim.x) {
@@ -695,7 +732,7 @@ cudaError_t launch_voxelize(const float* P, int64_t nv, const uint32_t* T, int64
     const uint32_t* Tc = T + 3 * t0;
     if (t0 > 0) cudaMemsetAsync(counts, 0, 2 * sizeof(uint32_t), st);
     GM_LAUNCH(kc, "k_vox_tris", st,
-              k_vox_tris<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(P, Tc, n, vp, list, counts));
+              k_vox_tris<<<(unsigned)((n + kVoxThreads - 1) / kVoxThreads), kVoxThreads, 0, st>>>(P, Tc, (uint32_t)n, vp, list, counts));
     const unsigned b = (unsigned)(n < 152 * 16 ? n : 152 * 16);
     GM_LAUNCH(kc, "k_vox_listed", st, k_vox_listed<<<b, 128, 0, st>>>(P, Tc, n, vp, list, counts));
   }
