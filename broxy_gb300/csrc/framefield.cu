@@ -32,9 +32,9 @@
 //     (res 256), so each round gains at least two digits, usually four.
 // Transforms are dense products along an axis, folded by the cosine
 // matrix's even and odd symmetry.  Two or three solutions of nine transform
-// kernels each replace thousands of conjugate-gradient iterations of six
-// dependent launches: 32^3 nodes, 4 constraints 124.9 -> 0.32 ms, and 2.6 ms
-// at 64^3, 35 ms at 128^3, 1.3 s at 256^3 with 20 constraints.
+// kernels (five on small lattices) each replace thousands of conjugate-gradient
+// iterations of six dependent launches: 32^3 nodes, 4 constraints 124.9 ->
+// 0.24 ms, and 1.6 ms at 64^3, 21 ms at 128^3; 1.3 s at 256^3 with 20.
 #include <math.h>
 
 #include <vector>
@@ -214,8 +214,149 @@ __global__ void __launch_bounds__(kFfThreads) k_ff_deg2(double* __restrict__ g, 
   g[i] = d * d;
 }
 
-__global__ void k_ff_units(double* __restrict__ HE, int nc, const __grid_constant__ FfPoints pts) {
-  if (threadIdx.x < pts.m) HE[(int64_t)pts.node[threadIdx.x] * nc + threadIdx.x] = 1.0;
+// The transforms of the unit vectors of the constrained nodes are products of
+// three cosines: the columns' forward transforms, their division by lambda
+// and the inverse along z in one kernel that reads nothing but the cosines.
+__global__ void __launch_bounds__(128) k_ff_units(double* __restrict__ v, int n, int nc, const double* __restrict__ C,
+                                                  const double* __restrict__ lam, double* __restrict__ dc,
+                                                  const __grid_constant__ FfPoints pts) {
+  extern __shared__ double ff_sm[];
+  double* a = ff_sm;
+  double* b = ff_sm + (size_t)n * kFfCols;
+  const int col = threadIdx.x & (kFfCols - 1), kg = threadIdx.x / kFfCols;
+  const int64_t inner = (int64_t)nc * n * n, q = (int64_t)blockIdx.x * kFfCols + col;
+  const bool ok = q < inner;
+  const int c = (int)(q % nc), kx = (int)((q / nc) % n), ky = (int)(q / ((int64_t)nc * n));
+  const bool on = ok && c < pts.m;
+  const int node = on ? pts.node[c] : 0, px = node % n, py = (node / n) % n, pz = node / (n * n);
+  const double cxy = on ? C[(size_t)kx * n + px] * C[(size_t)ky * n + py] : 0.0, lxy = on ? lam[kx] + lam[ky] : 0.0;
+  for (int k = kg; k < n; k += 8) {
+    double s = on ? cxy * C[(size_t)k * n + pz] : 0.0;
+    if (ok && (kx | ky | k) == 0) {
+      dc[c] = s;  // the sum over the nodes / n^1.5
+      s = 0.0;
+    } else if (on) {
+      s /= lxy + lam[k];
+    }
+    b[k * kFfCols + col] = s;
+  }
+  __syncthreads();
+  ff_inverse(C, n, b, a, col, kg);
+  if (ok)
+    for (int i = kg; i < n; i += 8) v[(int64_t)i * inner + q] = a[i * kFfCols + col];
+}
+
+// ---- transforms of an xy plane
+//
+// On small lattices a launch per axis waits longer than it computes: a block
+// takes one plane of one component whole in shared memory, with the cosines,
+// through what lies between two transforms along z:
+//   FF_FWD: along x and y; FF_INV: inverse along both;
+//   FF_WEIGHT: inverse along both, multiply by deg^2, along both
+// (16 warps; lane: the line, warp: wave number or element mod 16.  E: ceil of
+// n / 16.)  Taken up to 32 nodes an axis, where a solve of 4 constraints went
+// from 0.317 to 0.243 ms (32) and 0.232 to 0.174 (16) together with
+// k_ff_units.  Above, the second round of lines leaves lanes idle and a plane
+// leaves an SM few blocks: 48: 0.78 ms with a launch per axis, 1.02 with
+// planes; 64: no difference.
+constexpr int kFfPlaneThreads = 512;
+
+// element i of line l at i es + l ls
+template <int E>
+__device__ __forceinline__ void plane_forward(const double* C, int n, double* src, double* dst, int es, int ls) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  for (int l = lane; l < n; l += 32)
+    for (int i = wid; i < n / 2; i += 16) {
+      double *p = src + i * es + l * ls, *q = src + (n - 1 - i) * es + l * ls;
+      const double a = *p, b = *q;
+      *p = a + b;
+      *q = a - b;
+    }
+  __syncthreads();
+  const bool odd = wid & 1;  // the parity of every wave number wid + 16 m
+  const int cnt = odd ? n / 2 : (n + 1) / 2, step = odd ? -es : es;
+  const double* row[E];
+#pragma unroll
+  for (int m = 0; m < E; m++) row[m] = C + (wid + 16 * m < n ? wid + 16 * m : 0) * n;
+  for (int l = lane; l < n; l += 32) {
+    const double* s = src + l * ls + (odd ? (n - 1) * es : 0);
+    double acc[E];
+#pragma unroll
+    for (int m = 0; m < E; m++) acc[m] = 0;
+    for (int i = 0; i < cnt; i++) {
+      const double x = s[i * step];
+#pragma unroll
+      for (int m = 0; m < E; m++) acc[m] = fma(row[m][i], x, acc[m]);
+    }
+#pragma unroll
+    for (int m = 0; m < E; m++)
+      if (wid + 16 * m < n) dst[(wid + 16 * m) * es + l * ls] = acc[m];
+  }
+  __syncthreads();
+}
+
+template <int E>
+__device__ __forceinline__ void plane_inverse(const double* C, int n, const double* src, double* dst, int es, int ls) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nh = (n + 1) / 2;
+  constexpr int H = (E + 1) / 2;  // elements of a half line a thread
+  for (int l = lane; l < n; l += 32) {
+    const double* s = src + l * ls;
+    double e[H], o[H];
+#pragma unroll
+    for (int m = 0; m < H; m++) e[m] = o[m] = 0;
+    for (int k = 0; k < n; k += 2) {
+      const double ye = s[k * es], yo = k + 1 < n ? s[(k + 1) * es] : 0.0;
+      const double *ce = C + k * n, *co = C + (k + 1 < n ? k + 1 : k) * n;
+#pragma unroll
+      for (int m = 0; m < H; m++) {
+        const int i = wid + 16 * m < nh ? wid + 16 * m : 0;
+        e[m] = fma(ce[i], ye, e[m]);
+        o[m] = fma(co[i], yo, o[m]);
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < H; m++) {
+      const int i = wid + 16 * m;
+      if (i < nh) {  // (the middle of an odd line: the odd wave numbers vanish there)
+        dst[(n - 1 - i) * es + l * ls] = e[m] - o[m];
+        dst[i * es + l * ls] = e[m] + o[m];
+      }
+    }
+  }
+  __syncthreads();
+}
+
+template <int MODE, int E>
+__global__ void __launch_bounds__(kFfPlaneThreads) k_ff_plane(double* __restrict__ v, int n, int nc,
+                                                              const double* __restrict__ cosines) {
+  extern __shared__ double ff_sm[];
+  const int pitch = n + 1;  // (lines along either axis without bank conflicts)
+  double* C = ff_sm;
+  double* a = C + n * n;
+  double* b = a + n * pitch;
+  const int z = (int)(blockIdx.x / nc), c = (int)(blockIdx.x % nc);
+  double* plane = v + (int64_t)z * n * n * nc + c;
+  for (int i = threadIdx.x; i < n * n; i += kFfPlaneThreads) {
+    C[i] = cosines[i];
+    a[i / n * pitch + i % n] = plane[(int64_t)i * nc];
+  }
+  __syncthreads();
+  if (MODE != FF_FWD) {
+    plane_inverse<E>(C, n, a, b, pitch, 1);
+    plane_inverse<E>(C, n, b, a, 1, pitch);
+  }
+  if (MODE == FF_WEIGHT) {
+    for (int i = threadIdx.x; i < n * n; i += kFfPlaneThreads) {
+      const double d = (double)ff_deg(i % n, i / n, z, n);
+      a[i / n * pitch + i % n] *= d * d;
+    }
+    __syncthreads();
+  }
+  if (MODE != FF_INV) {
+    plane_forward<E>(C, n, a, b, 1, pitch);
+    plane_forward<E>(C, n, b, a, pitch, 1);
+  }
+  for (int i = threadIdx.x; i < n * n; i += kFfPlaneThreads) plane[(int64_t)i * nc] = a[i / n * pitch + i % n];
 }
 
 // ---- the small dense correction (one block)
@@ -504,19 +645,53 @@ cudaError_t ff_line(FrameFieldGpu& f, double* v, int axis, int nc, double* dc, c
   return cudaGetLastError();
 }
 
-// v = G^+ D^2 G^+ v without beta, the sums' coefficients into dc[0 .. nc)
-// (of v) and dc[nc ..) (of D^2 G^+ v)
-cudaError_t ff_h0(FrameFieldGpu& f, double* v, int nc, double* dc, cudaStream_t st, KernelCounter* kc) {
+// the transforms of an xy plane of MODE (see k_ff_plane), one launch or one per axis
+template <int MODE, int E>
+cudaError_t ff_plane_e(FrameFieldGpu& f, double* v, int nc, cudaStream_t st, KernelCounter* kc) {
+  const int n = f.res;
+  const size_t smem = sizeof(double) * ((size_t)n * n + 2 * (size_t)n * (n + 1));
+  cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(k_ff_plane<MODE, E>), smem);
+  if (e != cudaSuccess) return e;
+  GM_LAUNCH(kc, "k_ff_plane", st,
+            k_ff_plane<MODE, E><<<(unsigned)(n * nc), kFfPlaneThreads, smem, st>>>(v, n, nc, f.cosines));
+  return cudaGetLastError();
+}
+template <int MODE>
+cudaError_t ff_plane(FrameFieldGpu& f, double* v, int nc, cudaStream_t st, KernelCounter* kc) {
+  const int n = f.res;
+  if (n <= 16) return ff_plane_e<MODE, 1>(f, v, nc, st, kc);
+  if (n <= 32) return ff_plane_e<MODE, 2>(f, v, nc, st, kc);
   cudaError_t e;
-  if ((e = ff_line<FF_FWD>(f, v, 0, nc, dc, st, kc)) != cudaSuccess) return e;
-  if ((e = ff_line<FF_FWD>(f, v, 1, nc, dc, st, kc)) != cudaSuccess) return e;
-  if ((e = ff_line<FF_SOLVE>(f, v, 2, nc, dc, st, kc)) != cudaSuccess) return e;
-  if ((e = ff_line<FF_INV>(f, v, 1, nc, dc, st, kc)) != cudaSuccess) return e;
-  if ((e = ff_line<FF_WEIGHT>(f, v, 0, nc, dc, st, kc)) != cudaSuccess) return e;
-  if ((e = ff_line<FF_FWD>(f, v, 1, nc, dc, st, kc)) != cudaSuccess) return e;
+  if (MODE == FF_FWD) {
+    if ((e = ff_line<FF_FWD>(f, v, 0, nc, nullptr, st, kc)) != cudaSuccess) return e;
+    return ff_line<FF_FWD>(f, v, 1, nc, nullptr, st, kc);
+  }
+  if ((e = ff_line<FF_INV>(f, v, 1, nc, nullptr, st, kc)) != cudaSuccess) return e;
+  if (MODE == FF_INV) return ff_line<FF_INV>(f, v, 0, nc, nullptr, st, kc);
+  if ((e = ff_line<FF_WEIGHT>(f, v, 0, nc, nullptr, st, kc)) != cudaSuccess) return e;
+  return ff_line<FF_FWD>(f, v, 1, nc, nullptr, st, kc);
+}
+
+// v = G^+ D^2 G^+ v without beta, the sums' coefficients into dc[0 .. nc)
+// (of v) and dc[nc ..) (of D^2 G^+ v); with pts, v starts as their nodes'
+// unit vectors (and need not hold anything)
+cudaError_t ff_h0(FrameFieldGpu& f, double* v, int nc, const FfPoints* pts, double* dc, cudaStream_t st,
+                  KernelCounter* kc) {
+  cudaError_t e;
+  if (pts) {
+    const int n = f.res;
+    const size_t smem = sizeof(double) * 2 * kFfCols * (size_t)n;
+    if ((e = ensure_dynamic_smem(reinterpret_cast<const void*>(k_ff_units), smem)) != cudaSuccess) return e;
+    GM_LAUNCH(kc, "k_ff_units", st,
+              k_ff_units<<<(unsigned)(((int64_t)n * n * nc + kFfCols - 1) / kFfCols), 128, smem, st>>>(
+                  v, n, nc, f.cosines, f.lambda, dc, *pts));
+  } else {
+    if ((e = ff_plane<FF_FWD>(f, v, nc, st, kc)) != cudaSuccess) return e;
+    if ((e = ff_line<FF_SOLVE>(f, v, 2, nc, dc, st, kc)) != cudaSuccess) return e;
+  }
+  if ((e = ff_plane<FF_WEIGHT>(f, v, nc, st, kc)) != cudaSuccess) return e;
   if ((e = ff_line<FF_SOLVE>(f, v, 2, nc, dc + nc, st, kc)) != cudaSuccess) return e;
-  if ((e = ff_line<FF_INV>(f, v, 1, nc, dc, st, kc)) != cudaSuccess) return e;
-  return ff_line<FF_INV>(f, v, 0, nc, dc, st, kc);
+  return ff_plane<FF_INV>(f, v, nc, st, kc);
 }
 
 // The field's plan, on its first solve: cosine matrix, eigenvalues, G^+ of
@@ -543,11 +718,9 @@ cudaError_t ff_plan(FrameFieldGpu& f, cudaStream_t st, KernelCounter* kc) {
     return e;
   if (!f.g && (e = cudaMalloc(&f.g, sizeof(double) * total)) != cudaSuccess) return e;
   GM_LAUNCH(kc, "k_ff_deg2", st, k_ff_deg2<<<ff_blocks(total), kFfThreads, 0, st>>>(f.g, n));
-  if ((e = ff_line<FF_FWD>(f, f.g, 0, 1, f.dc, st, kc)) != cudaSuccess) return e;
-  if ((e = ff_line<FF_FWD>(f, f.g, 1, 1, f.dc, st, kc)) != cudaSuccess) return e;
+  if ((e = ff_plane<FF_FWD>(f, f.g, 1, st, kc)) != cudaSuccess) return e;
   if ((e = ff_line<FF_SOLVE>(f, f.g, 2, 1, f.dc, st, kc)) != cudaSuccess) return e;
-  if ((e = ff_line<FF_INV>(f, f.g, 1, 1, f.dc, st, kc)) != cudaSuccess) return e;
-  if ((e = ff_line<FF_INV>(f, f.g, 0, 1, f.dc, st, kc)) != cudaSuccess) return e;
+  if ((e = ff_plane<FF_INV>(f, f.g, 1, st, kc)) != cudaSuccess) return e;
   // sum of deg^2 over the lattice: end nodes of an axis count 1, others 2
   f.sum_deg2 = 0;
   for (int ends = 0; ends < 8; ends++) {
@@ -636,9 +809,7 @@ cudaError_t frame_field_solve(FrameFieldGpu& f, const int64_t* nodes, const floa
   FfSmall* sm = reinterpret_cast<FfSmall*>(f.small);
   const double dc_to_sum = (double)n * sqrt((double)n), dc_to_beta = -dc_to_sum / f.sum_deg2;
   // the columns H0 E and the first solution
-  if ((e = cudaMemsetAsync(f.HE, 0, sizeof(double) * total * nc, st)) != cudaSuccess) return e;
-  GM_LAUNCH(kc, "k_ff_units", st, k_ff_units<<<1, 32, 0, st>>>(f.HE, nc, pts));
-  if ((e = ff_h0(f, f.HE, nc, f.dc, st, kc)) != cudaSuccess) return e;
+  if ((e = ff_h0(f, f.HE, nc, &pts, f.dc, st, kc)) != cudaSuccess) return e;
   GM_LAUNCH(kc, "k_ff_small", st, k_ff_small_first<<<1, 512, 0, st>>>(f.HE, nc, f.g, f.dc + nc, dc_to_beta, pts, sm));
   GM_LAUNCH(kc, "k_ff_apply", st,
             k_ff_apply<true><<<nb, kFfThreads, 0, st>>>(f.x, nullptr, f.HE, nc, pts.m, f.g, sm, total));
@@ -655,7 +826,7 @@ cudaError_t frame_field_solve(FrameFieldGpu& f, const int64_t* nodes, const floa
         if (f.h_rr[k] > tol * tol * bb[k]) done = false;
       if (done || rounds >= kFfMaxRounds) break;
     }
-    if ((e = ff_h0(f, f.r, 4, f.dc, st, kc)) != cudaSuccess) return e;
+    if ((e = ff_h0(f, f.r, 4, nullptr, f.dc, st, kc)) != cudaSuccess) return e;
     GM_LAUNCH(kc, "k_ff_small", st,
               k_ff_small<<<1, 128, 0, st>>>(f.r, f.g, f.dc, f.dc + 4, dc_to_sum, dc_to_beta, pts, sm));
     GM_LAUNCH(kc, "k_ff_apply", st,

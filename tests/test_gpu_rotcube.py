@@ -267,6 +267,24 @@ def test_frame_field_sizes(gm_ctx, qres, npts):
     ff.destroy()
 
 
+def test_frame_field_by_lines(gm_ctx):
+    """The first lattice past those transformed by planes; constraints in
+    corners, on a face and inside."""
+    import torch
+    qres = 33
+    pts = [((0.0, 0.0, 0.0), (0.3, 0.1, -0.2)), ((0.99, 0.99, 0.99), (-0.5, 0.2, 0.4)), ((0.4, 0.99, 0.7), (0.1, 0.9, 0.0)),
+           ((0.52, 0.31, 0.63), (0.0, -0.4, 0.8))]
+    ff = api.FrameField(gm_ctx, (0, 0, 0), (1, 1, 1), qres)
+    for pos, tw in pts:
+        ff.add_point(pos, tw)
+    ff.generate()
+    got = ff.quats().cpu().numpy()
+    torch.cuda.synchronize()
+    want = F.generate(qres, (0, 0, 0), (1, 1, 1), pts)
+    assert np.abs(got - want).max() <= 1e-5 * np.abs(want).max()
+    ff.destroy()
+
+
 def test_frame_field_same_node_last_wins(gm_ctx):
     """Two constraints on one lattice node: S is set once and b takes the
     later point's quaternion (FrameFieldSparseBiharmonic.cu:353-364,
