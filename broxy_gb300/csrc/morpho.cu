@@ -1495,7 +1495,7 @@ cudaError_t kernel_error_flags(unsigned int* flags, bool clear) {
 // every 8th of the 256 rows, so the block streams its 16 x 16 rows of the
 // field front to back, eight 16-byte loads a lane in flight.  With d_rmax, the
 // largest clamped radius is folded into *d_rmax as well.  Bound by the bytes
-// it reads: 0.149 ms for 1024^3 (7.2 TB/s; 0.24 with two rows in flight and
+// it reads: 0.150 ms for 1024^3 (7.2 TB/s; 0.172 with two rows in flight and
 // bytewise maxima), and 23 instead of 32 us for 64 x 512 x 512.
 constexpr int kRmapCells = 4;  // map cells per lane along x, at most
 
