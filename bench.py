@@ -134,7 +134,7 @@ LIMITER = {
 
 # ALU pipe utilisation of the min-plus passes from their ncu capture
 # (sm__pipe_alu_cycles_active, profiles/k_pass_dpx_512.md, 512^3 case).
-ALU_PIPE_NCU = {"k_pass_dil_y": 0.691, "k_pass_dil_z": 0.735}
+ALU_PIPE_NCU = {"k_pass_dil_y": 0.787, "k_pass_dil_z": 0.790, "k_pass_ero_y": 0.769, "k_pass_ero_z": 0.801}
 
 
 # DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) from
