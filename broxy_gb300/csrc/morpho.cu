@@ -716,7 +716,10 @@ __global__ void __launch_bounds__(256) k_final_z_base(const uint16_t* __restrict
 // value + kernel never wraps in 16 bits.
 //   FIN 0: write the u16 field;  FIN 1: dilation threshold + packed bytes;
 //   FIN 2: erosion threshold (centres) + packed bytes;
-//   FIN 3: erosion threshold at lattice points 2c+1, one flag per cell.
+//   FIN 3: erosion threshold at lattice points 2c+1, one flag per cell;
+//   FIN 4: FIN 2's bytes e applied to the closing (out8): a cell tagged 0xff
+//          in the tags, handed over in R.p, becomes ~e, the others stay (a
+//          kernel of its own for it took 14.6 us at 512^3, 47 at 1024^3).
 // ---------------------------------------------------------------------
 
 constexpr int kDpxCols = 64;   // x columns per block
@@ -905,6 +908,7 @@ __device__ __forceinline__ void dpx_tile(const TIn* __restrict__ in, uint16_t* _
   // passes feeding them within their window): a tile outside writes its
   // saturation value ("not eroded") without work.
   const bool needed = tile_needed(need, axis, sub, o0, nout, bx, bz);
+  if (FIN == 4 && !needed) return;  // (block-uniform; no tagged cell)
   const int skip = needed ? halo - halo_e : span;  // tile rows never read
   const uint32_t capp = cap | (cap << 16);
   uint32_t* tile = tileu + tpar * span * 32;
@@ -1175,10 +1179,20 @@ __device__ __forceinline__ void dpx_tile(const TIn* __restrict__ in, uint16_t* _
     if (tpar == 0 && colok && obase < nout) {
       bytes[0] |= xch[grp][lane][0];
       bytes[1] |= xch[grp][lane][1];
-      uint8_t* dst = out8 + idx3(x >> 1, third >> 1, obase / 2, rx, ry);
+      const int64_t o = idx3(x >> 1, third >> 1, obase / 2, rx, ry);
+      uint8_t* dst = out8 + o;
 #pragma unroll
-      for (int q = 0; q < kDpxPer / 2; q++)
-        dst[(int64_t)rx * ry * q] = (uint8_t)((bytes[q >> 2] >> (8 * (q & 3))) & 0xffu);
+      for (int q = 0; q < kDpxPer / 2; q++) {
+        const uint32_t e = (bytes[q >> 2] >> (8 * (q & 3))) & 0xffu;
+        if (FIN == 4) {
+          // (tags exist in groups of 16 cells along x that meet the region)
+          const int cx = x >> 1, cy = third >> 1, cz = obase / 2 + q;
+          if (cbox_meets(need.roi, cx & ~15, cx | 15, cy, cy, cz, cz) && R.p[o + (int64_t)rx * ry * q] != 0)
+            dst[(int64_t)rx * ry * q] = (uint8_t)~e;
+        } else {
+          dst[(int64_t)rx * ry * q] = (uint8_t)e;
+        }
+      }
     }
   }
 }
@@ -1244,6 +1258,7 @@ enum DpxKind {
   DPXK_CUBE_U16_1,     // cube dilation z
   DPXK_CEN2_U16_0,     // centre erosion y
   DPXK_CEN2_U16_2,     // centre erosion z
+  DPXK_CEN2_U16_4,     // the same, applied to the closing (GM_REF)
   DPXK_LAT2_U16_0,     // lattice-point erosion y
   DPXK_LAT2_U16_3,     // lattice-point erosion z
   DPXK_COUNT
@@ -1256,6 +1271,7 @@ constexpr int dpx_kind() {
          : G == KERN_CUBE && sizeof(TIn) == 2 && FIN == 1 ? DPXK_CUBE_U16_1
          : G == KERN_CEN2 && sizeof(TIn) == 2 && FIN == 0 ? DPXK_CEN2_U16_0
          : G == KERN_CEN2 && sizeof(TIn) == 2 && FIN == 2 ? DPXK_CEN2_U16_2
+         : G == KERN_CEN2 && sizeof(TIn) == 2 && FIN == 4 ? DPXK_CEN2_U16_4
          : G == KERN_LAT2 && sizeof(TIn) == 2 && FIN == 0 ? DPXK_LAT2_U16_0
          : G == KERN_LAT2 && sizeof(TIn) == 2 && FIN == 3 ? DPXK_LAT2_U16_3
                                                           : -1;
@@ -1406,7 +1422,7 @@ static bool dpx_record(DpxGroup* grp, const TIn* in, uint16_t* out16, uint8_t* o
 
 static const char* const kDpxGroupNames[DPXK_COUNT] = {
     "k_pass_dil_y_group", "k_pass_dil_z_group",  "k_pass_dil_y_group",  "k_pass_dil_z_group",
-    "k_pass_ero_y_group", "k_pass_ero_z_group", "k_pass_erob_y_group", "k_pass_erob_z_group"};
+    "k_pass_ero_y_group", "k_pass_ero_z_group", "k_pass_ero_z_group", "k_pass_erob_y_group", "k_pass_erob_z_group"};
 
 template <int G, typename TIn, int FIN>
 static cudaError_t dpx_group_go(DpxGroup* g, int sms, cudaStream_t st, KernelCounter* kc) {
@@ -1447,6 +1463,7 @@ cudaError_t dpx_group_launch(DpxGroup* g, int sms, cudaStream_t st, KernelCounte
     case DPXK_CUBE_U16_1: return dpx_group_go<KERN_CUBE, uint16_t, 1>(g, sms, st, kc);
     case DPXK_CEN2_U16_0: return dpx_group_go<KERN_CEN2, uint16_t, 0>(g, sms, st, kc);
     case DPXK_CEN2_U16_2: return dpx_group_go<KERN_CEN2, uint16_t, 2>(g, sms, st, kc);
+    case DPXK_CEN2_U16_4: return dpx_group_go<KERN_CEN2, uint16_t, 4>(g, sms, st, kc);
     case DPXK_LAT2_U16_0: return dpx_group_go<KERN_LAT2, uint16_t, 0>(g, sms, st, kc);
     case DPXK_LAT2_U16_3: return dpx_group_go<KERN_LAT2, uint16_t, 3>(g, sms, st, kc);
     default: return cudaErrorInvalidValue;
@@ -1819,10 +1836,13 @@ __device__ __forceinline__ void base_dil_row(const uint8_t* X, const uint8_t* Df
 // The select kernel computes each base-pass row once: a block walks along z,
 // each thread keeping its row's flags at z and z + 1 in registers; the row
 // y + 1 comes from the block's next row of threads through shared memory (its
-// last row is that halo only).
+// last row is that halo only).  It marks the 8^3-cell blocks of D that hold a
+// non-zero byte in dmap (zeroed by the caller; reading D again for them took
+// 12.5 us at 512^3, 63 at 1024^3).
 __global__ void __launch_bounds__(kWalkThreads) k_dil_select_z(const uint8_t* __restrict__ X,
                                                                const uint8_t* __restrict__ Df, uint8_t* __restrict__ D,
-                                                               Dims g, int zs, DataRes dr, CBox roi) {
+                                                               Dims g, int zs, DataRes dr, CBox roi,
+                                                               uint8_t* __restrict__ dmap, int mdx, int mdy) {
   __shared__ uint4 flags_s[4][kWalkThreads];  // per thread: f, fr at z; f, fr at z + 1
   const int bx = blockDim.x, ty = threadIdx.y, me = ty * bx + threadIdx.x;
   const int x16 = 16 * (blockIdx.x * bx + threadIdx.x);
@@ -1839,6 +1859,7 @@ __global__ void __launch_bounds__(kWalkThreads) k_dil_select_z(const uint8_t* __
     }
   };
   uint32_t d0c[4], fc[4], frc[4], dfc[4];
+  uint32_t seen0 = 0, seen1 = 0;  // of the two 8-cell blocks along x, since the last mark
   row(z0, d0c, fc, frc, dfc);
   for (int z = z0; z < z1; z++) {
     uint32_t d0n[4], fn[4], frn[4], dfn[4];
@@ -1862,6 +1883,14 @@ __global__ void __launch_bounds__(kWalkThreads) k_dil_select_z(const uint8_t* __
         o[j] = (tag & dfc[j]) | (~tag & d0c[j]);
       }
       *reinterpret_cast<uint4*>(D + cidx(x16, y, z, g)) = make_uint4(o[0], o[1], o[2], o[3]);
+      seen0 |= o[0] | o[1];
+      seen1 |= o[2] | o[3];
+    }
+    if ((z & 7) == 7 || z == z1 - 1) {
+      uint8_t* m = dmap + idx3(x16 >> 3, y >> 3, z >> 3, mdx, mdy);
+      if (seen0) m[0] = 1;
+      if (seen1) m[1] = 1;
+      seen0 = seen1 = 0;
     }
     __syncthreads();  // flags_s is rewritten for the next z
 #pragma unroll
@@ -1949,12 +1978,12 @@ __global__ void __launch_bounds__(256) k_ero_select16(const uint8_t* __restrict_
 
 static dim3 grid16(Dims g) { return dim3((g.x / 16 + 31) / 32, (g.y + 7) / 8, g.z); }
 
-// GM_REF erosion select in two steps, so that the centre erosion Ef is
-// computed only where it is read.  k_ero_tag_z writes the base erosion C0
-// into C (final for untagged cells), the refinement tags (0xff per tagged
-// cell) into T and marks the 8^3-cell blocks holding a tagged cell in tmap
-// (zeroed by the caller); once Ef is known on those blocks, k_ero_fix16
-// writes 0xff & ~Ef on the tagged cells.  The bytes equal k_ero_select16's.
+// GM_REF erosion select in two steps, so that the centre erosion is computed
+// only where it is read.  k_ero_tag_z writes the base erosion C0 into C (final
+// for untagged cells), the refinement tags (0xff per tagged cell) into T and
+// marks the 8^3-cell blocks holding a tagged cell in tmap (zeroed by the
+// caller); the centre erosion's z pass then runs on those blocks and writes
+// 0xff & ~e on the tagged cells.  The bytes equal k_ero_select16's.
 // The tag kernel computes each base-erosion row once: a block walks along z,
 // each thread keeping its row's C0 at z - 1, z, z + 1 in registers; the rows
 // y - 1 and y + 1 at z come from the block's other threads through shared
@@ -2033,27 +2062,6 @@ __global__ void __launch_bounds__(kWalkThreads) k_ero_tag_z(const uint8_t* __res
     }
   }
 }
-
-__global__ void __launch_bounds__(256) k_ero_fix16(const uint8_t* __restrict__ T, const uint8_t* __restrict__ Ef,
-                                                   uint8_t* __restrict__ C, Dims g, CBox roi) {
-  const int x16 = 16 * (blockIdx.x * 32 + threadIdx.x);
-  const int y = blockIdx.y * 8 + threadIdx.y, z = blockIdx.z;
-  if (x16 >= g.x || y >= g.y || !cbox_meets(roi, x16, x16 + 15, y, y, z, z)) return;
-  const int64_t o = cidx(x16, y, z, g);
-  const uint4 t = *reinterpret_cast<const uint4*>(T + o);
-  if ((t.x | t.y | t.z | t.w) == 0u) return;
-  const uint4 e = *reinterpret_cast<const uint4*>(Ef + o);
-  uint4 c = *reinterpret_cast<const uint4*>(C + o);
-  c.x = (t.x & ~e.x) | (~t.x & c.x);
-  c.y = (t.y & ~e.y) | (~t.y & c.y);
-  c.z = (t.z & ~e.z) | (~t.z & c.z);
-  c.w = (t.w & ~e.w) | (~t.w & c.w);
-  *reinterpret_cast<uint4*>(C + o) = c;
-}
-
-
-
-
 
 // max clamped radius over the fine radius grid
 __global__ void k_rmax(const int8_t* __restrict__ R, int64_t n, int* __restrict__ out) {
@@ -2297,14 +2305,17 @@ cudaError_t launch_close(const CloseArgs& a, cudaStream_t st, KernelCounter* kc)
     }
     if (!exact && here()) {
       const ZWalk w = z_walk(g, 1);
+      cudaMemsetAsync(dmap, 0, (size_t)(tmap - dmap) + (size_t)mdx * mdy * mdz, st);  // both block maps
       GM_LAUNCH(kc, "k_dil_select", st,
-                k_dil_select_z<<<w.blocks, w.threads, 0, st>>>(a.X, Df, D, g, w.zs, dr, R_D));
+                k_dil_select_z<<<w.blocks, w.threads, 0, st>>>(a.X, Df, D, g, w.zs, dr, R_D, dmap, mdx, mdy));
     }
   } else {
     at += 2;  // the dilation's two passes
   }
   // ---- occupancy map of D (erosion outputs are needed on D only) ----
-  if (here()) {
+  // (k_dil_select has marked it already)
+  const bool mapped = !exact && !a.dilation_done;
+  if (!mapped && here()) {
     const int nb = mdx * mdy * mdz;
     GM_LAUNCH(kc, "k_occ_map8", st, k_occ_map8<<<(nb + 7) / 8, 256, 0, st>>>(D, rx, ry, mdx, mdy, nb, dmap));
   }
@@ -2346,7 +2357,7 @@ cudaError_t launch_close(const CloseArgs& a, cudaStream_t st, KernelCounter* kc)
         // any more: it holds the tags), then the centre erosion only on the
         // blocks of tagged cells (ero y within the z window of them)
         if (here()) {
-          cudaMemsetAsync(tmap, 0, (size_t)mdx * mdy * mdz, st);
+          if (!mapped) cudaMemsetAsync(tmap, 0, (size_t)mdx * mdy * mdz, st);
           const ZWalk w = z_walk(g, 2);
           GM_LAUNCH(kc, "k_ero_tag", st,
                     k_ero_tag_z<<<w.blocks, w.threads, 0, st>>>(a.X, D, Eb, a.C_out, S, tmap, mdx, mdy, g, w.zs, dr, F));
@@ -2354,11 +2365,10 @@ cudaError_t launch_close(const CloseArgs& a, cudaStream_t st, KernelCounter* kc)
         ok &= dpx_step<KERN_CEN2, uint16_t, 0>(a, at, buf16a, buf16b, nullptr, Nx, Ny, Nz, 1, 0, ehalo, K, RNONE, 0, rx,
                                                ry, st, kc, "k_pass_ero_y", nullptr, 0,
                                                NeedMap{tmap, mdx, mdy, mdz, 1, 1, 0, 0, gz, B_ero_y});
-        ok &= dpx_step<KERN_CEN2, uint16_t, 2>(a, at, buf16b, nullptr, Ef, Nx, Ny, Nz, 2, 0, ehalo, K, RNONE, 0, rx, ry,
-                                               st, kc, "k_pass_ero_z", nullptr, 0,
+        ok &= dpx_step<KERN_CEN2, uint16_t, 4>(a, at, buf16b, nullptr, a.C_out, Nx, Ny, Nz, 2, 0, ehalo, K,
+                                               RField{reinterpret_cast<const int8_t*>(S), 0, 0}, 0, rx, ry, st, kc,
+                                               "k_pass_ero_z", nullptr, 0,
                                                NeedMap{tmap, mdx, mdy, mdz, 1, 1, 0, 0, 0, R_Ef});
-        if (here())
-          GM_LAUNCH(kc, "k_ero_fix", st, k_ero_fix16<<<grid16(g), dim3(32, 8), 0, st>>>(S, Ef, a.C_out, g, F));
       }
       if (!ok) return cudaErrorInvalidValue;
     } else {
