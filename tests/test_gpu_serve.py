@@ -235,3 +235,18 @@ def test_admission_by_memory_failures_and_timeout(gm_ctx):
     assert srv.memory()[0] == 0
     assert len(ran) >= 1
     srv.destroy()
+
+
+def test_crops_at_every_offset(gm_ctx):
+    """Brushes a cell apart along x, one after the other: their crops and dirty
+    boxes start and end at every residue of the copies' 16-byte pieces."""
+    import torch
+    cs = 0.5 / 128
+    edits = [(np.array([0.4 + 2 * i * cs, 0.5 + 2 * (i % 3) * cs, 0.5]), (5 + i % 4) * cs,
+              (5 + i % 4) * cs + 4.0 * cs * np.sqrt(1 - np.sqrt(0.5)), L.GM_BRUSH_MAX) for i in range(17)]
+    desc, X, R, C, results, srv = _run(1, edits)
+    assert all(r["status"] == L.GM_OK for r in results)
+    full = gm_ctx.close(desc, X, R, 0, L.GM_REF, L.GM_SE_SPHERE)
+    torch.cuda.synchronize()
+    assert torch.equal(C, full)
+    srv.destroy()
