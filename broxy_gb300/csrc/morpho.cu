@@ -1595,13 +1595,15 @@ __global__ void __launch_bounds__(256) k_radius_map(RField R, int mbx, int mby, 
 cudaError_t launch_radius_map(RField R, int nx, int ny, int nz, uint8_t* out, int* d_rmax, cudaStream_t st,
                               KernelCounter* kc) {
   const int mbx = nx / 16, mby = ny / 16, mbz = nz / 16;
-  if (mbx > 32 * kRmapCells) return cudaErrorInvalidValue;
+  if (!radius_map_takes(nx)) return cudaErrorInvalidValue;
   const int aligned = ((uintptr_t)R.p % 16 == 0 && R.sy % 16 == 0 && R.sz % 16 == 0) ? 1 : 0;
   if (d_rmax) cudaMemsetAsync(d_rmax, 0, sizeof(int), st);
   auto* kernel = mbx <= 32 ? k_radius_map<1> : (mbx <= 64 ? k_radius_map<2> : k_radius_map<kRmapCells>);
   GM_LAUNCH(kc, "k_radius_map", st, kernel<<<dim3(mby, mbz), 256, 0, st>>>(R, mbx, mby, aligned, out, d_rmax));
   return cudaGetLastError();
 }
+
+bool radius_map_takes(int nx) { return nx / 16 <= 32 * kRmapCells; }
 
 cudaError_t launch_radius_map_dense(const int8_t* R, int nx, int ny, int nz, uint8_t* out, int* d_rmax,
                                     cudaStream_t st, KernelCounter* kc) {
