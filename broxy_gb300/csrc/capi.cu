@@ -565,19 +565,13 @@ static gm_status close_box_impl(gm_ctx* ctx, const gm_box_desc* box, const uint8
   const uint8_t* rmap = nullptr;
   if (d_scale) {
     // one pass over the field gives its bound and the map of the tiles' bounds
-    // (rows wider than the map kernel takes: the bound alone)
-    if (gm::radius_map_takes(2 * rx)) {
-      if ((s = ensure(ctx, (void**)&ctx->rmap, ctx->rmap_bytes, (size_t)8 * rx * ry * rz / 4096 + 16,
-                      "radius map")) != GM_OK)
-        return s;
-      GM_CHECK_CUDA(ctx, gm::launch_radius_map_dense(d_scale, 2 * rx, 2 * ry, 2 * rz, ctx->rmap, ctx->d_int, st,
-                                                     &ctx->kc),
-                    "radius bound");
-      rmap = ctx->rmap;
-    } else {
-      GM_CHECK_CUDA(ctx, gm::launch_rmax(d_scale, (int64_t)8 * rx * ry * rz, ctx->d_int, ctx->num_sms, st, &ctx->kc),
-                    "radius bound");
-    }
+    if ((s = ensure(ctx, (void**)&ctx->rmap, ctx->rmap_bytes, (size_t)8 * rx * ry * rz / 4096 + 16, "radius map")) !=
+        GM_OK)
+      return s;
+    GM_CHECK_CUDA(ctx, gm::launch_radius_map_dense(d_scale, 2 * rx, 2 * ry, 2 * rz, ctx->rmap, ctx->d_int, st,
+                                                   &ctx->kc),
+                  "radius bound");
+    rmap = ctx->rmap;
     int h = 0;
     GM_CHECK_CUDA(ctx, cudaMemcpyAsync(&h, ctx->d_int, sizeof(int), cudaMemcpyDeviceToHost, st), "radius bound");
     GM_CHECK_CUDA(ctx, cudaStreamSynchronize(st), "radius bound");

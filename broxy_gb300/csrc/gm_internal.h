@@ -214,8 +214,7 @@ cudaError_t launch_edt(const uint8_t* X, int res, int rmax, uint8_t* workspace, 
 cudaError_t launch_rmax(const int8_t* R, int64_t n, int* d_out, int sms, cudaStream_t st, KernelCounter* kc);
 // The 16^3-block map of the largest raw radius of a dense field of nx*ny*nz
 // fine voxels ((nx/16)(ny/16)(nz/16) bytes), and its largest clamped radius
-// into *d_rmax (when given).  Rows of up to 2048 voxels (radius_map_takes).
-bool radius_map_takes(int nx);
+// into *d_rmax (when given).
 cudaError_t launch_radius_map_dense(const int8_t* R, int nx, int ny, int nz, uint8_t* out, int* d_rmax,
                                     cudaStream_t st, KernelCounter* kc);
 

@@ -1506,15 +1506,16 @@ cudaError_t kernel_error_flags(unsigned int* flags, bool clear) {
 }
 
 // Largest raw radius (>= 0) of each 16^3 block of fine voxels of a radius
-// field (nx, ny, nz multiples of 16, nx <= 16 * 32 * kRmapCells).  One block
-// per (map y, map z) row of map cells; a warp reads whole fine rows (lane l
-// owns the 16-byte segments of map cells l, l + 32, ...), the 8 warps take
-// every 8th of the 256 rows, so the block streams its 16 x 16 rows of the
-// field front to back, eight 16-byte loads a lane in flight.  With d_rmax, the
-// largest clamped radius is folded into *d_rmax as well.  Bound by the bytes
-// it reads: 0.150 ms for 1024^3 (7.2 TB/s; 0.172 with two rows in flight and
-// bytewise maxima), and 23 instead of 32 us for 64 x 512 x 512.
-constexpr int kRmapCells = 4;  // map cells per lane along x, at most
+// field (nx, ny, nz multiples of 16).  One block per (map y, map z) row of
+// map cells (per 32 * CELLS of them where the rows are longer, blockIdx.z); a
+// warp reads whole fine rows (lane l owns the 16-byte segments of map cells
+// l, l + 32, ...), the 8 warps take every 8th of the 256 rows, so the block
+// streams its 16 x 16 rows of the field front to back, eight 16-byte loads a
+// lane in flight.  With d_rmax, the largest clamped radius is folded into
+// *d_rmax as well.  Bound by the bytes it reads: 0.150 ms for 1024^3 (7.2
+// TB/s; 0.172 with two rows in flight and bytewise maxima), and 23 instead of
+// 32 us for 64 x 512 x 512.
+constexpr int kRmapCells = 4;  // map cells per lane along x, at most (registers and shared memory)
 
 // maxima of signed bytes, in 16-bit halves whose upper byte counts (the one
 // below it decides between equals only): the odd bytes, and the even ones
@@ -1532,6 +1533,8 @@ __global__ void __launch_bounds__(256) k_radius_map(RField R, int mbx, int mby, 
                                                      uint8_t* __restrict__ out, int* __restrict__ d_rmax) {
   const int my = blockIdx.x, mz = blockIdx.y;
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int c0 = 32 * CELLS * (int)blockIdx.z, n = min(mbx - c0, 32 * CELLS);  // the block's map cells
+  R.p += 16 * c0;
   __shared__ int part[8][32 * CELLS];
   int m[CELLS];
 #pragma unroll
@@ -1550,7 +1553,7 @@ __global__ void __launch_bounds__(256) k_radius_map(RField R, int mbx, int mby, 
 #pragma unroll
         for (int c = 0; c < CELLS; c++) {
           const int cx = lane + 32 * c;
-          v[k][c] = cx < mbx ? __ldcs(reinterpret_cast<const uint4*>(row + 16 * cx)) : make_uint4(0u, 0u, 0u, 0u);
+          v[k][c] = cx < n ? __ldcs(reinterpret_cast<const uint4*>(row + 16 * cx)) : make_uint4(0u, 0u, 0u, 0u);
         }
       }
 #pragma unroll
@@ -1569,7 +1572,7 @@ __global__ void __launch_bounds__(256) k_radius_map(RField R, int mbx, int mby, 
 #pragma unroll
       for (int c = 0; c < CELLS; c++) {
         const int cx = lane + 32 * c;
-        if (cx < mbx)
+        if (cx < n)
 #pragma unroll
           for (int j = 0; j < 16; j++) m[c] = max(m[c], (int)row[16 * cx + j]);
       }
@@ -1579,14 +1582,14 @@ __global__ void __launch_bounds__(256) k_radius_map(RField R, int mbx, int mby, 
   for (int c = 0; c < CELLS; c++) part[wid][lane + 32 * c] = m[c];
   __syncthreads();
   int gmax = 0;
-  for (int cx = threadIdx.x; cx < mbx; cx += blockDim.x) {
+  for (int cx = threadIdx.x; cx < n; cx += blockDim.x) {
     int t = 0;
 #pragma unroll
     for (int k = 0; k < 8; k++) t = max(t, part[k][cx]);
-    out[cx + (int64_t)mbx * (my + (int64_t)mby * mz)] = (uint8_t)t;
+    out[c0 + cx + (int64_t)mbx * (my + (int64_t)mby * mz)] = (uint8_t)t;
     gmax = max(gmax, t);
   }
-  if (d_rmax != nullptr && wid * 32 < mbx) {
+  if (d_rmax != nullptr && wid * 32 < n) {
     for (int o = 16; o > 0; o >>= 1) gmax = max(gmax, __shfl_xor_sync(0xffffffffu, gmax, o));
     if (lane == 0) atomicMax(d_rmax, clamp_radius(gmax));
   }
@@ -1595,15 +1598,13 @@ __global__ void __launch_bounds__(256) k_radius_map(RField R, int mbx, int mby, 
 cudaError_t launch_radius_map(RField R, int nx, int ny, int nz, uint8_t* out, int* d_rmax, cudaStream_t st,
                               KernelCounter* kc) {
   const int mbx = nx / 16, mby = ny / 16, mbz = nz / 16;
-  if (!radius_map_takes(nx)) return cudaErrorInvalidValue;
   const int aligned = ((uintptr_t)R.p % 16 == 0 && R.sy % 16 == 0 && R.sz % 16 == 0) ? 1 : 0;
   if (d_rmax) cudaMemsetAsync(d_rmax, 0, sizeof(int), st);
   auto* kernel = mbx <= 32 ? k_radius_map<1> : (mbx <= 64 ? k_radius_map<2> : k_radius_map<kRmapCells>);
-  GM_LAUNCH(kc, "k_radius_map", st, kernel<<<dim3(mby, mbz), 256, 0, st>>>(R, mbx, mby, aligned, out, d_rmax));
+  const int parts = (mbx + 32 * kRmapCells - 1) / (32 * kRmapCells);
+  GM_LAUNCH(kc, "k_radius_map", st, kernel<<<dim3(mby, mbz, parts), 256, 0, st>>>(R, mbx, mby, aligned, out, d_rmax));
   return cudaGetLastError();
 }
-
-bool radius_map_takes(int nx) { return nx / 16 <= 32 * kRmapCells; }
 
 cudaError_t launch_radius_map_dense(const int8_t* R, int nx, int ny, int nz, uint8_t* out, int* d_rmax,
                                     cudaStream_t st, KernelCounter* kc) {
