@@ -2235,6 +2235,7 @@ cudaError_t launch_close(const CloseArgs& a, cudaStream_t st, KernelCounter* kc)
   // phase mode: the steps of phase a.phase only (see CloseArgs::phase)
   if (a.phase >= 0 && (a.edt != nullptr || !close_phase_ok(rmax, a.se) || a.group == nullptr))
     return cudaErrorInvalidValue;
+  cudaError_t e;  // (the launchers of a pass report and clear the errors so far)
   int at = 0;  // min-plus passes met so far
   auto here = [&]() { return a.phase < 0 || a.phase == at; };
 
@@ -2251,8 +2252,7 @@ cudaError_t launch_close(const CloseArgs& a, cudaStream_t st, KernelCounter* kc)
     } else if (a.R != nullptr && a.rmap_in != nullptr) {
       tile_map = a.rmap_in;  // built by the caller together with the radius bound
     } else if (a.R != nullptr) {
-      if (here() && launch_radius_map(RF, Nx, Ny, Nz, rmap, nullptr, st, kc) != cudaSuccess)
-        return cudaGetLastError();
+      if (here() && (e = launch_radius_map(RF, Nx, Ny, Nz, rmap, nullptr, st, kc)) != cudaSuccess) return e;
       tile_map = rmap;
     }
     if (a.edt != nullptr) {
@@ -2260,8 +2260,9 @@ cudaError_t launch_close(const CloseArgs& a, cudaStream_t st, KernelCounter* kc)
                 k_dil_threshold<<<quad_grid(g), dim3(64, 4), 0, st>>>(a.edt, a.e_sy, a.e_sz, RF, a.uniform_r, g,
                                                                       exact ? D : Df, R_Df));
     } else {
-      if (!a.xpass_done && here() && launch_dil_pass_x(a.X, buf8, rx, ry, rz, dcap, B_dil_x, st, kc) != cudaSuccess)
-        return cudaGetLastError();
+      if (!a.xpass_done && here() &&
+          (e = launch_dil_pass_x(a.X, buf8, rx, ry, rz, dcap, B_dil_x, st, kc)) != cudaSuccess)
+        return e;
       uint8_t* dst = exact ? D : Df;
       if ((a.ypass_done || a.zpass_done) && a.se != 0) return cudaErrorInvalidValue;
       if (dil_cap <= 32767) {
@@ -2334,8 +2335,9 @@ cudaError_t launch_close(const CloseArgs& a, cudaStream_t st, KernelCounter* kc)
   {
     const uint32_t K = 4u * (uint32_t)((rmax - 1) * (rmax - 1));
     const int ehalo = rmax + 1;
-    if (here() && launch_ero_pass_x(S, RF, a.uniform_r, rx, ry, rz, ehalo, K, buf16a, HL1, B_ero_x, st, kc) != cudaSuccess)
-      return cudaGetLastError();
+    if (here() &&
+        (e = launch_ero_pass_x(S, RF, a.uniform_r, rx, ry, rz, ehalo, K, buf16a, HL1, B_ero_x, st, kc)) != cudaSuccess)
+      return e;
     if (K <= 32767) {
       const int gz = (ehalo + 1) / 2 + 1;  // cells covering the z window (ehalo fine voxels) of a z pass
       bool ok = true;
@@ -2422,8 +2424,8 @@ cudaError_t launch_edt(const uint8_t* X, int res, int rmax, uint8_t* workspace, 
   const int dil_r = rmax + 1, dil_halo = dil_r + 1, dcap = dil_r + 1;
   const uint32_t dil_cap = (uint32_t)(dil_r * dil_r);
   const RField RNONE{nullptr, 0, 0};
-  if (launch_dil_pass_x(X, buf8, res, res, res, dcap, CBox{{0, 0, 0}, {res, res, res}}, st, kc) != cudaSuccess)
-    return cudaGetLastError();
+  const cudaError_t e = launch_dil_pass_x(X, buf8, res, res, res, dcap, CBox{{0, 0, 0}, {res, res, res}}, st, kc);
+  if (e != cudaSuccess) return e;
   launch_dpx<KERN_LAT, uint8_t, 0>(buf8, buf16a, nullptr, N, N, N, 1, 0, dil_halo, dil_cap, RNONE, 0, res, res, st,
                                    kc, "k_pass_dil_y");
   launch_dpx<KERN_LAT, uint16_t, 0>(buf16a, E, nullptr, N, N, N, 2, 0, dil_halo, dil_cap, RNONE, 0, res, res, st,
