@@ -530,10 +530,9 @@ cudaError_t batch_run(void** state, int n, const gm_batch_item* it, int mode, in
   uint64_t sig = signature(n, it, ext, mode, se, L);
   if (meshes) {
     sig = mix(sig, (uint64_t)(uintptr_t)b->h_tot);
-    for (int i = 0; i < n; i++) {
-      sig = mix(sig, (uint64_t)(uintptr_t)b->meshes[i].brick_tot);
-      sig = mix(sig, (uint64_t)(uintptr_t)b->meshes[i].cells);
-    }
+    // (the scratch of the counting kernels, all of it: its addresses alone
+    // may come back after it was freed and allocated anew)
+    for (int i = 0; i < n; i++) sig = mix(sig, b->meshes[i].grid_moves);
   }
   const bool graphable = all_uniform && !(kc && kc->profiling);
   if (graphable) {

@@ -281,6 +281,7 @@ struct MeshBuffers {
   int64_t entries_cap = 0, n_cells = 0;
   uint32_t* fix = nullptr;        // case-91 fix list: 1 + 4 * fix_cap
   int64_t cells_cap = 0, bricks_cap = 0;
+  uint64_t grid_moves = 0;        // times that scratch was re-allocated
   int fix_cap = 0, n_fix = 0;
 };
 

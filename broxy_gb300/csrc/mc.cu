@@ -1218,6 +1218,7 @@ static McWin window_of(const MeshArgs& a) {
 // capacity helpers: buffers grow (never shrink) to the sizes asked for
 static cudaError_t ensure_grid_buffers(MeshBuffers& b, int64_t cells, int nb) {
   cudaError_t e;
+  if (nb + 1 > b.bricks_cap || cells > b.cells_cap) b.grid_moves++;
   if (nb + 1 > b.bricks_cap) {
     cudaFree(b.brick_tot);
     cudaFree(b.brick_mask);

@@ -2,7 +2,9 @@
 // (an executable that includes it takes them over from libcudart): launches
 // do nothing and are counted, device memory is host memory, copies copy. A
 // test can make a launch fail, and it can see when a captured graph is
-// replayed after memory that was there at its capture has been freed.
+// replayed after memory that was there at its capture has been freed.  Freed
+// memory is given out again, the longest free first, separately for requests
+// of up to 64 KB and for larger ones: addresses come back as from a device.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -10,6 +12,8 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <deque>
+#include <map>
 #include <set>
 
 namespace fake {
@@ -25,17 +29,30 @@ struct Graph {
 inline std::set<Graph*> instances;
 inline bool capturing = false;
 
+constexpr size_t kSmall = 64 << 10, kLarge = 512 << 20;  // (pages nobody touches cost nothing)
+inline std::map<void*, bool> small;
+inline std::deque<void*> unused[2];
+
 inline cudaError_t alloc(void** p, size_t n) {
-  *p = malloc(n ? n : 1);
+  *p = nullptr;
+  if (n > kLarge) return cudaErrorMemoryAllocation;
+  const bool s = n <= kSmall;
+  if (!unused[s].empty()) {
+    *p = unused[s].front();
+    unused[s].pop_front();
+  } else if ((*p = malloc(s ? kSmall : kLarge)) == nullptr) {
+    return cudaErrorMemoryAllocation;
+  }
+  small[*p] = s;
   live.insert(*p);
-  return *p ? cudaSuccess : cudaErrorMemoryAllocation;
+  return cudaSuccess;
 }
 inline cudaError_t release(void* p) {
   if (!p) return cudaSuccess;
   for (Graph* g : instances)
     if (g->memory.count(p)) g->stale = true;
   live.erase(p);
-  free(p);
+  unused[small[p]].push_back(p);
   return cudaSuccess;
 }
 inline cudaError_t launch() {
