@@ -74,6 +74,7 @@ struct BatchState {
   cudaEvent_t ev_in = nullptr, ev_out = nullptr;
   cudaGraphExec_t graph = nullptr;
   uint64_t graph_sig = 0;
+  uint64_t moves = 0;  // times that a workspace or table which a graph may name was re-allocated
   long long graph_kernels = 0;
   std::map<uint64_t, int> tuned;
   int last_tuned = 0;  // the form chosen by the latest tuning
@@ -306,6 +307,7 @@ static cudaError_t ensure_arena(BatchState* b, int n, const gm_batch_item* it, c
   }
   cudaError_t e;
   if (b->arena_bytes < total) {
+    b->moves++;
     cudaFree(b->arena);
     b->arena = nullptr;
     b->arena_bytes = 0;
@@ -320,8 +322,10 @@ static cudaError_t ensure_arena(BatchState* b, int n, const gm_batch_item* it, c
   for (auto& gs : b->groups)
     while ((int)gs.size() < P) gs.push_back(dpx_group_new());
   for (auto& gs : b->groups)
-    for (int p = 0; p < P; p++)
+    for (int p = 0; p < P; p++) {
+      if (dpx_group_room(gs[p]) < n) b->moves++;
       if ((e = dpx_group_reserve(gs[p], n)) != cudaSuccess) return e;
+    }
   return cudaSuccess;
 }
 
@@ -432,6 +436,7 @@ cudaError_t batch_run(void** state, int n, const gm_batch_item* it, int mode, in
   for (int l = 0; l < (L == kBatchGrouped ? 0 : maxL); l++) {
     BatchLane& ln = b->lanes[l];
     if (ln.ws_bytes < wsb) {
+      b->moves++;
       cudaFree(ln.ws);
       ln.ws = nullptr;
       ln.ws_bytes = 0;
@@ -439,6 +444,7 @@ cudaError_t batch_run(void** state, int n, const gm_batch_item* it, int mode, in
       ln.ws_bytes = wsb;
     }
     if (ln.crop_cells < ccells) {
+      b->moves++;
       cudaFree(ln.Xc);
       cudaFree(ln.Cc);
       ln.Xc = ln.Cc = nullptr;
@@ -526,8 +532,9 @@ cudaError_t batch_run(void** state, int n, const gm_batch_item* it, int mode, in
     }
   }
   // closing phase (with the mesh counts): replay the captured graph when the
-  // batch is unchanged
-  uint64_t sig = signature(n, it, ext, mode, se, L);
+  // batch is unchanged and the memory it names has not been re-allocated by
+  // another batch meanwhile
+  uint64_t sig = mix(signature(n, it, ext, mode, se, L), b->moves);
   if (meshes) {
     sig = mix(sig, (uint64_t)(uintptr_t)b->h_tot);
     // (the scratch of the counting kernels, all of it: its addresses alone

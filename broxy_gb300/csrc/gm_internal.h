@@ -65,8 +65,10 @@ DpxGroup* dpx_group_new();
 void dpx_group_free(DpxGroup* g);
 void dpx_group_clear(DpxGroup* g);
 int dpx_group_size(const DpxGroup* g);
-// Room for `njobs` grids (allocates; not while a stream is being captured).
+// Room for `njobs` grids (allocates; not while a stream is being captured);
+// more than dpx_group_room moves its tables.
 cudaError_t dpx_group_reserve(DpxGroup* g, int njobs);
+int dpx_group_room(const DpxGroup* g);
 // Uploads the recorded grids' pass arguments and launches one kernel whose
 // resident blocks pull the tiles of all of them from one work counter.
 cudaError_t dpx_group_launch(DpxGroup* g, int sms, cudaStream_t st, KernelCounter* kc);

@@ -1361,6 +1361,8 @@ void dpx_group_clear(DpxGroup* g) {
 
 int dpx_group_size(const DpxGroup* g) { return (int)g->jobs.size(); }
 
+int dpx_group_room(const DpxGroup* g) { return g->cap; }
+
 cudaError_t dpx_group_reserve(DpxGroup* g, int njobs) {
   if (njobs <= g->cap) return cudaSuccess;
   cudaError_t e;
