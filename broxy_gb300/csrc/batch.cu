@@ -361,6 +361,7 @@ cudaError_t batch_run(void** state, int n, const gm_batch_item* it, int mode, in
     if (b->h_rmax) cudaFreeHost(b->h_rmax);
     b->d_rmax = nullptr;
     b->h_rmax = nullptr;
+    b->rmax_cap = 0;
     if ((e = cudaMalloc(&b->d_rmax, sizeof(int) * n)) != cudaSuccess) return e;
     if ((e = cudaMallocHost(&b->h_rmax, sizeof(int) * n)) != cudaSuccess) return e;
     b->rmax_cap = n;
@@ -370,6 +371,7 @@ cudaError_t batch_run(void** state, int n, const gm_batch_item* it, int mode, in
     if (b->h_ext) cudaFreeHost(b->h_ext);
     b->d_ext = nullptr;
     b->h_ext = nullptr;
+    b->ext_cap = 0;
     if ((e = cudaMalloc(&b->d_ext, sizeof(unsigned) * 3 * n)) != cudaSuccess) return e;
     if ((e = cudaMallocHost(&b->h_ext, sizeof(unsigned) * 3 * n)) != cudaSuccess) return e;
     b->ext_cap = n;
@@ -502,6 +504,7 @@ cudaError_t batch_run(void** state, int n, const gm_batch_item* it, int mode, in
     if (b->h_tot_cap < n) {
       if (b->h_tot) cudaFreeHost(b->h_tot);
       b->h_tot = nullptr;
+      b->h_tot_cap = 0;
       if ((e = cudaMallocHost(&b->h_tot, sizeof(uint32_t) * 4 * n)) != cudaSuccess) return e;
       b->h_tot_cap = n;
     }

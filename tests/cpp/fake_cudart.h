@@ -1,7 +1,7 @@
 // A stand-in for the CUDA runtime calls that the library's host code makes
 // (an executable that includes it takes them over from libcudart): launches
 // do nothing and are counted, device memory is host memory, copies copy. A
-// test can make a launch fail, and it can see when a captured graph is
+// test can make a launch or an allocation fail, and it can see when a captured graph is
 // replayed after memory that was there at its capture has been freed.  Freed
 // memory is given out again, the longest free first, separately for requests
 // of up to 64 KB and for larger ones: addresses come back as from a device.
@@ -19,6 +19,7 @@
 namespace fake {
 inline cudaError_t last = cudaSuccess;
 inline long launches = 0, fail_at = -1;      // the launch with this number fails
+inline long allocs = 0, fail_alloc_at = -1;  // the allocation with this number fails
 inline int graphs = 0, stale_replays = 0;    // captures so far; replays of graphs whose memory was freed
 inline uint32_t read_back = 0;               // every device-to-host copy gives these words
 inline std::set<void*> live;
@@ -35,7 +36,7 @@ inline std::deque<void*> unused[2];
 
 inline cudaError_t alloc(void** p, size_t n) {
   *p = nullptr;
-  if (n > kLarge) return cudaErrorMemoryAllocation;
+  if (allocs++ == fail_alloc_at || n > kLarge) return cudaErrorMemoryAllocation;
   const bool s = n <= kSmall;
   if (!unused[s].empty()) {
     *p = unused[s].front();
@@ -65,7 +66,9 @@ cudaError_t handle(T* out) {
   *out = reinterpret_cast<T>(next += 16);
   return cudaSuccess;
 }
+inline int null_copies = 0;  // copies and fills at a null pointer
 inline cudaError_t copy(void* dst, const void* src, size_t n, cudaMemcpyKind kind) {
+  if (!dst || !src) return null_copies++, cudaSuccess;
   if (kind != cudaMemcpyDeviceToHost) {
     if (kind == cudaMemcpyHostToDevice) memcpy(dst, src, n);
     return cudaSuccess;
@@ -99,7 +102,7 @@ cudaError_t cudaFreeHost(void* p) { return fake::release(p); }
 cudaError_t cudaMemcpyAsync(void* dst, const void* src, size_t n, cudaMemcpyKind kind, cudaStream_t) {
   return fake::copy(dst, src, n, kind);
 }
-cudaError_t cudaMemsetAsync(void*, int, size_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaMemsetAsync(void* p, int, size_t, cudaStream_t) { return fake::null_copies += !p, cudaSuccess; }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) { return fake::handle(s); }
 cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
