@@ -99,6 +99,7 @@ PROTOTYPES = {
     "gm_mesh_download": (C.c_int, [_P, _P, _P, _P, _P]),
     "gm_batch_close_mesh": (C.c_int, [_P, C.c_int32, C.POINTER(BatchItem), C.c_int, C.c_int, C.c_int32, C.c_int32,
                                        C.POINTER(MeshView), _P]),
+    "gm_mesh_inject_filter_stalls": (C.c_int, [_P, C.c_int32]),
     "gm_batch_lanes": (C.c_int32, [_P]),
     "gm_batch_inject_alloc_failures": (C.c_int, [_P, C.c_int32]),
     "gm_server_create": (C.c_int, [C.POINTER(GridDesc), _P, _P, C.POINTER(ServerOpts), C.POINTER(_P)]),

@@ -30,7 +30,8 @@ class DevicePtrArray:
 
 def kernel_error_flags(clear=False):
     """Error bits this library's kernels recorded on the current device
-    (bit 0: a kernel's bounded wait ran out; no kernel waits at present)."""
+    (bit 0: the barrier of a small mesh's normal filter ran out, and the
+    normals of that mesh are NaN)."""
     f = C.c_uint32(0)
     L.check(None, L.load().gm_kernel_error_flags(C.byref(f), 1 if clear else 0))
     return int(f.value)

@@ -133,6 +133,8 @@ struct gm_ctx {
   cudaEvent_t ev_slab[kSlabs] = {}, ev_max[kSlabs] = {};
   int* h_slab = nullptr;
   // last mesh
+  uint32_t* h_gave_up = nullptr;  // pinned: its normal filter's barrier ran out
+  int stall_filters = 0;          // filters still to stall (fault injection)
   gm::MeshBuffers mesh;
   int64_t nv = 0, nt = 0;
   bool has_mesh = false;
@@ -184,6 +186,21 @@ gm_status ensure(gm_ctx* ctx, void** p, size_t& have, size_t need, const char* w
   return GM_OK;
 }
 
+// Before a mesh's emission (its counting has waited for the stream, so no
+// earlier filter is at work): the word that its filter may set.
+void arm_filter(gm_ctx* ctx, gm::MeshArgs& a) {
+  *ctx->h_gave_up = 0;
+  a.gave_up = ctx->h_gave_up;
+  a.stall_filter = ctx->stall_filters > 0;
+  if (a.stall_filter) ctx->stall_filters--;
+}
+
+// After the mesh's stream has been waited for.
+gm_status filter_status(gm_ctx* ctx, const char* where) {
+  if (*static_cast<volatile uint32_t*>(ctx->h_gave_up) == 0) return GM_OK;
+  return fail(ctx, GM_ERR_CUDA, std::string(where) + ": the normal filter's barrier ran out, normals are NaN");
+}
+
 gm_status set_device(gm_ctx* ctx) {
   GM_CHECK_CUDA(ctx, cudaSetDevice(ctx->device), "cudaSetDevice");
   return GM_OK;
@@ -220,6 +237,12 @@ gm_status gm_ctx_create(int device, gm_ctx** out) {
   if (cudaSetDevice(device) != cudaSuccess) { delete c; return GM_ERR_CUDA; }
   cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, device);
   if (cudaMalloc(&c->d_int, 16 * sizeof(int)) != cudaSuccess) { delete c; return GM_ERR_OUT_OF_MEMORY; }
+  if (cudaMallocHost(&c->h_gave_up, sizeof(uint32_t)) != cudaSuccess) {
+    cudaFree(c->d_int);
+    delete c;
+    return GM_ERR_OUT_OF_MEMORY;
+  }
+  *c->h_gave_up = 0;
   *out = c;
   return GM_OK;
 }
@@ -243,6 +266,7 @@ gm_status gm_ctx_destroy(gm_ctx* ctx) {
   }
   if (ctx->h_slab) cudaFreeHost(ctx->h_slab);
   ctx->mesh.release();
+  cudaFreeHost(ctx->h_gave_up);  // (the frees above have waited for the device)
   gm::batch_release(ctx->batch);
   ctx->kc.release();
   delete ctx;
@@ -667,6 +691,7 @@ gm_status gm_mesh_box(gm_ctx* ctx, const gm_box_desc* box, const uint8_t* d_clos
   GM_CHECK_CUDA(ctx, gm::mesh_count(a, ctx->mesh, st, &ctx->kc, &nv, &nt), "gm_mesh_box (count)");
   if (nv > 0xfffffff0LL || nt > 0x7ffffff0LL)
     return fail(ctx, GM_ERR_CAPACITY, "gm_mesh_box: mesh exceeds 32-bit vertex/triangle indexing");
+  arm_filter(ctx, a);
   GM_CHECK_CUDA(ctx, gm::mesh_emit(a, ctx->mesh, nv, nt, st, &ctx->kc), "gm_mesh_box (emit)");
   ctx->nv = nv;
   ctx->nt = nt;
@@ -697,6 +722,7 @@ static gm_status mesh_impl(gm_ctx* ctx, const gm_grid_desc* desc, const uint8_t*
   GM_CHECK_CUDA(ctx, gm::mesh_count(a, ctx->mesh, st, &ctx->kc, &nv, &nt), "gm_mesh (count)");
   if (nv > 0xfffffff0LL || nt > 0x7ffffff0LL)
     return fail(ctx, GM_ERR_CAPACITY, "gm_mesh: mesh exceeds 32-bit vertex/triangle indexing");
+  arm_filter(ctx, a);
   GM_CHECK_CUDA(ctx, gm::mesh_emit(a, ctx->mesh, nv, nt, st, &ctx->kc), "gm_mesh (emit)");
   ctx->nv = nv;
   ctx->nt = nt;
@@ -881,7 +907,7 @@ static gm_status update_impl(gm_ctx* ctx, const gm_grid_desc* desc, const uint8_
     GM_CHECK_CUDA(ctx, cudaMemcpyAsync(h_N, ctx->mesh.N, 12 * (size_t)ctx->nv, cudaMemcpyDeviceToHost, st), "D2H");
   GM_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->copy_st), "gm_update_to_host");
   GM_CHECK_CUDA(ctx, cudaStreamSynchronize(st), "gm_update_to_host");
-  return GM_OK;
+  return filter_status(ctx, "gm_update_to_host");
 }
 
 gm_status gm_update(gm_ctx* ctx, const gm_grid_desc* desc, const uint8_t* h_input, const int8_t* h_scale,
@@ -923,6 +949,12 @@ gm_status gm_mesh_download(gm_ctx* ctx, float* h_V, float* h_N, uint32_t* h_T, v
   if (h_T && ctx->nt)
     GM_CHECK_CUDA(ctx, cudaMemcpyAsync(h_T, ctx->mesh.T, 12 * (size_t)ctx->nt, cudaMemcpyDeviceToHost, st), "D2H");
   GM_CHECK_CUDA(ctx, cudaStreamSynchronize(st), "gm_mesh_download");
+  return filter_status(ctx, "gm_mesh_download");
+}
+
+gm_status gm_mesh_inject_filter_stalls(gm_ctx* ctx, int32_t count) {
+  if (!ctx || count < 0) return GM_ERR_INVALID_ARGUMENT;
+  ctx->stall_filters = count;
   return GM_OK;
 }
 

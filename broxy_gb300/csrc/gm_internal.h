@@ -257,6 +257,11 @@ struct MeshArgs {
   // mesh_emit stops after the vertex normals and the bilateral entries:
   // the caller runs the filtering (mesh_filter_group, several meshes at once)
   bool defer_filter = false;
+  // Pinned word that mesh_emit's kernels set when the filter's barrier ran out
+  // (its blocks' normals are NaN then); the caller clears it before mesh_emit
+  // and reads it once the stream's work is done.
+  uint32_t* gave_up = nullptr;
+  bool stall_filter = false;  // fault injection: that barrier waits for an arrival too many, briefly
 };
 
 // Device-side mesh buffers, grown on demand by the caller of launch_mesh.

@@ -1046,16 +1046,20 @@ __global__ void k_bilateral(const float4* __restrict__ Nin, const uint2* __restr
 // zeroes the counter before it).  The acquire of the count and the block
 // barrier after it order the other blocks' normals before the plain loads of
 // the next iteration.  The blocks are resident together, so the wait ends, and
-// it gives up after kResPolls polls all the same (an error bit).
+// it gives up after `polls` polls all the same: an error bit, a word that the
+// host reads after it has waited for the kernel (gave_up), and NaN normals for
+// the block's vertices.  (missing: arrivals that never come, for tests.)
 constexpr int kResGathers = 8;
 constexpr int kResThreads = 1024;  // at most; one block per SM, so that few arrive
-constexpr uint32_t kResPolls = 1u << 24;
+constexpr uint32_t kResPolls = 1u << 24, kResPollsStalled = 1u << 12;
 
 __global__ void __launch_bounds__(kResThreads) k_bilateral_resident(float4* Na, float4* Nb,
                                                                     const uint2* __restrict__ rec,
                                                                     const uint32_t* __restrict__ roff, uint32_t nv,
                                                                     int iters, int zero_isolated, uint32_t* arrived,
-                                                                    float* __restrict__ N3, unsigned int* errors) {
+                                                                    uint32_t missing, uint32_t polls,
+                                                                    float* __restrict__ N3, unsigned int* errors,
+                                                                    uint32_t* gave_up) {
   extern __shared__ uint32_t mine_s[];  // [2 kResGathers][threads]: the first records' neighbours, then terms
   const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x, pitch = blockDim.x;
   uint32_t* mine = mine_s + threadIdx.x;
@@ -1104,17 +1108,26 @@ __global__ void __launch_bounds__(kResThreads) k_bilateral_resident(float4* Na, 
     __syncthreads();
     int ok = 1;
     if (threadIdx.x == 0) {
-      const uint32_t want = (uint32_t)(it + 1) * gridDim.x;
+      const uint32_t want = (uint32_t)(it + 1) * gridDim.x + missing;
       __threadfence();  // the block's normals before its arrival
       atomicAdd(arrived, 1u);
-      uint32_t seen, polls = 0;
+      uint32_t seen, left = polls;
       do {
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(arrived) : "memory");
-        ok = ++polls < kResPolls;
-      } while (seen < want && ok);
-      if (!ok) atomicOr(errors, 1u);
+      } while (seen < want && --left);
+      if (seen < want) {
+        ok = 0;
+        atomicOr(errors, 1u);
+        if (gave_up) *reinterpret_cast<volatile uint32_t*>(gave_up) = 1u;
+      }
     }
-    if (!__syncthreads_and(ok)) return;
+    if (!__syncthreads_and(ok)) {
+      if (v < nv) {
+        float* o = N3 + 3 * (size_t)v;
+        o[0] = o[1] = o[2] = __int_as_float(0x7fffffff);
+      }
+      return;
+    }
   }
 }
 
@@ -1401,9 +1414,11 @@ cudaError_t mesh_emit(const MeshArgs& a, MeshBuffers& b, int64_t nv, int64_t nt,
   const int res_threads = (int)(share < 128 ? 128 : share);
   if (iters > 1 && res_threads <= kResThreads) {
     uint32_t nv32 = (uint32_t)nv, *arrived = counters + kCntArrived;
+    uint32_t missing = a.stall_filter ? 1u : 0u, polls = a.stall_filter ? kResPollsStalled : kResPolls;
+    uint32_t* gave_up = a.gave_up;
     unsigned int* errors = kernel_error_word();
     void* args[] = {&b.N4a, &b.N4b, &b.rec, &b.roff, &nv32, const_cast<int*>(&iters), const_cast<int*>(&zi),
-                    &arrived, &b.N, &errors};
+                    &arrived, &missing, &polls, &b.N, &errors, &gave_up};
     const size_t res_smem = 2 * kResGathers * sizeof(uint32_t) * (size_t)res_threads;
     cudaError_t le = ensure_dynamic_smem(reinterpret_cast<const void*>(k_bilateral_resident), res_smem);
     if (le != cudaSuccess) return le;

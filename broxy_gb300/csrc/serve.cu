@@ -86,7 +86,7 @@ struct Slot {
   cudaStream_t st = nullptr;
   cudaEvent_t t0 = nullptr, t1 = nullptr, counted = nullptr;
   cudaEvent_t written = nullptr;  // the edit's closing is in the resident grid (later overlapping edits wait on it)
-  uint32_t* h_tot = nullptr;  // pinned: the crop mesh's four totals
+  uint32_t* h_tot = nullptr;  // pinned: the crop mesh's four totals, then whether its filter gave up
   int phase = 0;              // 0 idle, 1 closing + counting, 2 emitting
   MeshArgs ma;
   uint8_t *Xc = nullptr, *Cc = nullptr, *ws = nullptr;  // carved from `block`
@@ -404,6 +404,8 @@ static cudaError_t dispatch(Server& s, Slot& sl, const Pending& p, const Plan& p
 static cudaError_t finish_mesh(Server& s, Slot& sl) {
   cudaError_t err;
   if ((err = mesh_count_finish(sl.mesh, sl.h_tot, &sl.nv, &sl.nt)) != cudaSuccess) return err;
+  sl.h_tot[4] = 0;
+  sl.ma.gave_up = sl.h_tot + 4;
   if ((err = mesh_emit(sl.ma, sl.mesh, sl.nv, sl.nt, sl.st, s.kc)) != cudaSuccess) return err;
   sl.phase = 2;
   cudaEventRecord(sl.t1, sl.st);
@@ -475,7 +477,8 @@ static void progress(Server& s) {
     if (q == cudaErrorNotReady) continue;
     gm_edit_result r;
     r.ticket = sl.ticket;
-    r.status = q == cudaSuccess ? GM_OK : GM_ERR_CUDA;
+    const bool gave_up = *static_cast<volatile uint32_t*>(sl.h_tot + 4) != 0;
+    r.status = q == cudaSuccess && !gave_up ? GM_OK : GM_ERR_CUDA;
     float dev_ms = 0.f;
     cudaEventElapsedTime(&dev_ms, sl.t0, sl.t1);
     r.device_ms = dev_ms;
@@ -658,7 +661,7 @@ gm_status gm_server_create(const gm_grid_desc* desc, const uint8_t* d_input, int
     if (e == cudaSuccess) e = cudaEventCreate(&sl.t1);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&sl.counted, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&sl.written, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaMallocHost(&sl.h_tot, 4 * sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMallocHost(&sl.h_tot, 5 * sizeof(uint32_t));
     // mesh buffers for a patch of a few surface layers across the largest
     // crop, so that the first large edits do not allocate
     const int64_t nt = 16 * (int64_t)s.max_cres * s.max_cres;

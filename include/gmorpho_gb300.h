@@ -91,10 +91,12 @@ const char* gm_ctx_last_error(const gm_ctx* ctx);
 /* number of this library's kernels launched on the context so far */
 long long gm_ctx_kernel_launches(const gm_ctx* ctx);
 /* Error bits that this library's kernels recorded on the current device
- * instead of trapping: bit 0 = a bounded wait of a kernel ran out (the
- * results of that call are not trustworthy; the grid barrier of the normal
- * filter on small meshes is the one that waits).  Waits for the device's
- * work; clears the bits when `clear`.
+ * instead of trapping: bit 0 = a bounded wait of a kernel ran out.  One
+ * kernel waits: the normal filter of small meshes, at a barrier over its
+ * grid; where that ran out, the mesh's filtered normals are NaN, and the
+ * calls that wait for a mesh (gm_update_to_host, gm_mesh_download, an edit's
+ * result) report GM_ERR_CUDA themselves.  Waits for the device's work;
+ * clears the bits when `clear`.
  * No counterpart in the reference (which checks cudaGetLastError only,
  * GMorpho/GMorpho.cu:50-56). */
 gm_status gm_kernel_error_flags(uint32_t* flags, int32_t clear);
@@ -247,7 +249,14 @@ gm_status gm_update_to_host(gm_ctx* ctx, const gm_grid_desc* desc, const uint8_t
                             float global_scale, const gm_update_opts* opts, float* h_V, float* h_N, uint32_t* h_T,
                             int64_t vertex_capacity, int64_t triangle_capacity, int64_t* num_vertices,
                             int64_t* num_triangles, void* stream);
+/* (GM_ERR_CUDA, with the arrays copied, where the mesh's normal filter ran
+ * out of polls: see gm_kernel_error_flags) */
 gm_status gm_mesh_download(gm_ctx* ctx, float* h_vertices, float* h_normals, uint32_t* h_triangles, void* stream);
+
+/* Fault injection for tests: the barrier of the next `count` meshes' normal
+ * filters on this context waits for one arrival more than will come, for a
+ * few milliseconds (meshes too large for that filter are not affected). */
+gm_status gm_mesh_inject_filter_stalls(gm_ctx* ctx, int32_t count);
 
 /* ---------------------------------------------------------------- batch */
 /* One instance of a batched closing: its own grid, radius and output. */
