@@ -712,11 +712,11 @@ cudaError_t ff_plan(FrameFieldGpu& f, cudaStream_t st, KernelCounter* kc) {
     c[(size_t)n * n + k] = 4.0 * s * s;  // 2 - 2 cos(pi k / n)
   }
   if (!f.cosines && (e = cudaMalloc(&f.cosines, sizeof(double) * c.size())) != cudaSuccess) return e;
+  if (!f.g && (e = cudaMalloc(&f.g, sizeof(double) * total)) != cudaSuccess) return e;
   f.lambda = f.cosines + (size_t)n * n;
   // (the copy reads pageable memory: it has left c when the call returns)
   if ((e = cudaMemcpyAsync(f.cosines, c.data(), sizeof(double) * c.size(), cudaMemcpyHostToDevice, st)) != cudaSuccess)
     return e;
-  if (!f.g && (e = cudaMalloc(&f.g, sizeof(double) * total)) != cudaSuccess) return e;
   GM_LAUNCH(kc, "k_ff_deg2", st, k_ff_deg2<<<ff_blocks(total), kFfThreads, 0, st>>>(f.g, n));
   if ((e = ff_plane<FF_FWD>(f, f.g, 1, st, kc)) != cudaSuccess) return e;
   if ((e = ff_line<FF_SOLVE>(f, f.g, 2, 1, f.dc, st, kc)) != cudaSuccess) return e;
@@ -797,7 +797,6 @@ cudaError_t frame_field_solve(FrameFieldGpu& f, const int64_t* nodes, const floa
   }
   for (int c = 0; c < pts.m; c++)
     for (int k = 0; k < 4; k++) bb[k] += pts.q[c][k] * pts.q[c][k];
-  if (!f.planned && (e = ff_plan(f, st, kc)) != cudaSuccess) return e;
   const int nc = (pts.m + 3) / 4 * 4;
   if (nc > f.HE_cols) {
     cudaFree(f.HE);
@@ -806,6 +805,9 @@ cudaError_t frame_field_solve(FrameFieldGpu& f, const int64_t* nodes, const floa
     if ((e = cudaMalloc(&f.HE, sizeof(double) * total * nc)) != cudaSuccess) return e;
     f.HE_cols = nc;
   }
+  // (all memory is there before the first launch: a solve that fails for
+  // memory leaves no plan at work on a stream that the next may not be on)
+  if (!f.planned && (e = ff_plan(f, st, kc)) != cudaSuccess) return e;
   FfSmall* sm = reinterpret_cast<FfSmall*>(f.small);
   const double dc_to_sum = (double)n * sqrt((double)n), dc_to_beta = -dc_to_sum / f.sum_deg2;
   // the columns H0 E and the first solution
