@@ -111,7 +111,7 @@ KERNEL_BYTES_PER_VOXEL = {
     "k_pass_dil_y": 1 + 2,                # u8 distances in, u16 partial sums out
     "k_pass_dil_z": 2 + 1 + 1 / 8,        # u16 in, radius in, packed dilation bits out
     "k_pass_ero_y": 2 + 2,                # u16 in, u16 out (voxel centres)
-    "k_pass_ero_z": 2 + 1 / 8,            # u16 in, packed eroded bits out
+    "k_pass_ero_z": 2 + 1 / 8,            # u16 in, refinement tags in (only tagged cells are written)
     "k_pass_erob_y": 1 + 0.5,             # lattice points 2c+1: (res, N, N) u16 in, (res, res, N) out
     "k_pass_erob_z": 0.5 + 1 / 8,         # (res, res, N) u16 in, one flag per cell out
     "k_ero_pass_x": 1 / 8 + 1 + 2 + 1,    # contour bits + radius in, centre + lattice fields out
@@ -134,15 +134,15 @@ LIMITER = {
 
 # ALU pipe utilisation of the min-plus passes from their ncu capture
 # (sm__pipe_alu_cycles_active, profiles/k_pass_dpx_512.md, 512^3 case).
-ALU_PIPE_NCU = {"k_pass_dil_y": 0.787, "k_pass_dil_z": 0.790, "k_pass_ero_y": 0.769, "k_pass_ero_z": 0.801}
+ALU_PIPE_NCU = {"k_pass_dil_y": 0.788, "k_pass_dil_z": 0.792, "k_pass_ero_y": 0.770, "k_pass_ero_z": 0.720}
 
 
 # DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) from
 # one ncu capture of each kernel, scaled to the 1024^3 workload by the
 # units processed (see profiles/).
 TRAFFIC = {
-    "k_bilateral": 550_000_000,     # 129.0 MB at 1.70M vertices / 3.40M triangles, x4.26
-    "k_pass_dil_z": 3_358_000_000,  # 419.7 MB at 512^3 fine voxels, x8
+    "k_bilateral": 539_000_000,     # 126.7 MB at 1.70M vertices / 3.40M triangles, x4.26
+    "k_pass_dil_z": 3_354_000_000,  # 419.3 MB at 512^3 fine voxels, x8
 }
 
 

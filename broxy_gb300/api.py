@@ -384,7 +384,8 @@ class FrameField:
         return tuple(g), tuple(t)
 
     def generate(self):
-        """Solve the field; returns the solver's iteration count."""
+        """Solve the field; returns the number of solutions taken (the first
+        and its refinements)."""
         it = C.c_int32()
         self.ctx._check(self.ctx.lib.gm_frame_field_generate(self.h, C.byref(it), _stream()))
         return it.value

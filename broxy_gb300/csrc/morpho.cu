@@ -25,7 +25,6 @@
 #include <string.h>
 
 #include <algorithm>
-#include <mutex>
 #include <vector>
 
 #include "gm_common.cuh"
@@ -1631,15 +1630,11 @@ __global__ void __launch_bounds__(256) k_occ_map8(const uint8_t* __restrict__ G,
 }
 
 // ---------------------------------------------------------------------
-// cell-level kernels
-// ---------------------------------------------------------------------
-
-struct DataRes { int v[3]; };
-
-// ---------------------------------------------------------------------
 // cell-level kernels; cell grids of this section are boxes of rx * ry * rz
 // cells (Dims), z = blockIdx.z
 // ---------------------------------------------------------------------
+
+struct DataRes { int v[3]; };
 
 struct Dims { int x, y, z; };
 __device__ __forceinline__ int64_t cidx(int x, int y, int z, Dims d) { return idx3(x, y, z, d.x, d.y); }

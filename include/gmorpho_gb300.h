@@ -188,9 +188,12 @@ gm_status gm_frame_field_get_point(const gm_frame_field* ff, int32_t i, float* g
  * degree-normalised 6-neighbour Laplacian (float entries as the reference
  * builds them), S the indicator of constrained nodes and b_k their
  * quaternions (sin(theta/2) axis, cos(theta/2)).  The reference factors the
- * system in float (sparse Cholesky); here conjugate gradients in double
- * until every residual is below 1e-10 |b_k|.  *iterations (may be NULL): the
- * iterations run.  Synchronises the stream. */
+ * system in float (sparse Cholesky); here a direct solution in double (cosine
+ * transforms, a dense correction for the constraints), refined on the real
+ * system until every residual is below 1e-10 |b_k|, at most 40 times.
+ * *iterations (may be NULL): the solutions taken, two or three as a rule.  A
+ * field's first solve also makes its plan and allocates res^3 * 8 bytes per
+ * constraint (rounded up to four).  Synchronises the stream. */
 gm_status gm_frame_field_generate(gm_frame_field* ff, int32_t* iterations, void* stream);
 /* The device quaternions ((x, y, z, w) floats per node, x-fastest; the
  * reference's quats_pong), valid until the next generate or destroy. */
