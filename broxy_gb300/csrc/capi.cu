@@ -20,7 +20,8 @@
 namespace gm {
 
 cudaError_t ensure_dynamic_smem(const void* kernel, size_t bytes) {
-  if (bytes <= 48 * 1024) return cudaSuccess;
+  // 48 KB hold a block's static shared memory as well (at most 1280 bytes here)
+  if (bytes <= 46 * 1024) return cudaSuccess;
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;

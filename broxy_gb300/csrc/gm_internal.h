@@ -36,7 +36,7 @@ struct KernelCounter {
 // Raises `kernel`'s dynamic shared memory limit to at least `bytes` on the
 // current device.  The attribute is per device, so the record of what was
 // set is kept per (kernel, device); safe to call from several host threads.
-// Needed only above the default 48 KB.
+// Needed only where that and the kernel's static shared memory exceed 48 KB.
 cudaError_t ensure_dynamic_smem(const void* kernel, size_t bytes);
 
 // The error bits kernels of this library recorded on the current device
