@@ -203,6 +203,7 @@ gm_status filter_status(gm_ctx* ctx, const char* where) {
 }
 
 gm_status set_device(gm_ctx* ctx) {
+  gm::drop_stale_error();
   GM_CHECK_CUDA(ctx, cudaSetDevice(ctx->device), "cudaSetDevice");
   return GM_OK;
 }

@@ -69,6 +69,7 @@ extern "C" gm_status gm_close_noalloc(const gm_grid_desc* desc, const uint8_t* d
   const size_t ws_offset = kRmaxSlotBytes + rmap_slot_bytes(res);
   if (ws_offset + gm::close_workspace_bytes(res) > kStaticScratchBytes) return GM_ERR_CAPACITY;
 
+  gm::drop_stale_error();
   cudaStream_t st = (cudaStream_t)stream;
   uint8_t* scratch = nullptr;
   int sms = 0;

@@ -46,6 +46,11 @@ cudaError_t kernel_error_flags(unsigned int* flags, bool clear);
 // Their device word, for the kernels of other files.
 unsigned int* kernel_error_word();
 
+// At every entry point that launches work: an error that an earlier call of
+// the program's own has left unread is not this call's (the launchers read the
+// last error; one that lasts comes back from the next call).
+inline void drop_stale_error() { cudaGetLastError(); }
+
 // JSON {"name": {"launches": n, "ms": t}, ...} of the counter's totals;
 // returns the bytes needed (with the terminating zero), copies when cap allows
 int64_t profile_json(KernelCounter& kc, char* buf, int64_t cap);

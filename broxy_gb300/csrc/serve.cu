@@ -600,6 +600,7 @@ gm_status gm_server_create(const gm_grid_desc* desc, const uint8_t* d_input, int
   if (opts->slots < 1 || opts->slots > 16 || !crop_ok || opts->max_crop_res > desc->res || opts->rmax < 2 ||
       opts->rmax > 127)
     return GM_ERR_INVALID_ARGUMENT;
+  gm::drop_stale_error();
   gm_server* srv = new gm_server();
   gm::Server& s = srv->s;
   cudaGetDevice(&s.device);
@@ -744,6 +745,7 @@ gm_status gm_server_submit(gm_server* srv, const gm_edit* edit, uint64_t* ticket
   gm::Pending p{srv->s.next_ticket++, *edit, gm::now_ms()};
   srv->s.queue.push_back(p);
   if (ticket) *ticket = p.ticket;
+  gm::drop_stale_error();
   cudaSetDevice(srv->s.device);
   gm::progress(srv->s);
   return GM_OK;
@@ -751,6 +753,7 @@ gm_status gm_server_submit(gm_server* srv, const gm_edit* edit, uint64_t* ticket
 
 gm_status gm_server_poll(gm_server* srv, gm_edit_result* results, int32_t cap, int32_t* count) {
   if (!srv || !count || (cap > 0 && !results)) return GM_ERR_INVALID_ARGUMENT;
+  gm::drop_stale_error();
   cudaSetDevice(srv->s.device);
   gm::progress(srv->s);
   int n = 0;
@@ -789,6 +792,7 @@ gm_status gm_server_restore(gm_server* srv, const uint8_t* h_closing, const int8
   if (!srv || !h_closing || !h_scale) return GM_ERR_INVALID_ARGUMENT;
   gm::Server& s = srv->s;
   if (gm_server_pending(srv) != 0) return GM_ERR_NOT_READY;
+  gm::drop_stale_error();
   cudaSetDevice(s.device);
   const size_t cells = (size_t)s.desc.res * s.desc.res * s.desc.res;
   cudaError_t e = cudaDeviceSynchronize();

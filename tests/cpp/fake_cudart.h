@@ -94,6 +94,10 @@ cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const
 }
 cudaError_t cudaGetSymbolAddress(void** p, const void* s) { return *p = const_cast<void*>(s), cudaSuccess; }
 cudaError_t cudaGetDevice(int* d) { return *d = 0, cudaSuccess; }
+cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+cudaError_t cudaGetDeviceCount(int* n) { return *n = 1, cudaSuccess; }
+cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int) { return *v = 152, cudaSuccess; }
+cudaError_t cudaDeviceSynchronize() { return cudaSuccess; }
 cudaError_t cudaMalloc(void** p, size_t n) { return fake::alloc(p, n); }
 cudaError_t cudaMallocHost(void** p, size_t n) { return fake::alloc(p, n); }
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { return fake::alloc(p, n); }
@@ -102,6 +106,15 @@ cudaError_t cudaFreeHost(void* p) { return fake::release(p); }
 cudaError_t cudaMemcpyAsync(void* dst, const void* src, size_t n, cudaMemcpyKind kind, cudaStream_t) {
   return fake::copy(dst, src, n, kind);
 }
+cudaError_t cudaMemcpy(void* dst, const void* src, size_t n, cudaMemcpyKind kind) { return fake::copy(dst, src, n, kind); }
+cudaError_t cudaMemset(void*, int, size_t) { return cudaSuccess; }
+cudaError_t cudaMemGetInfo(size_t* f, size_t* t) { return *f = *t = (size_t)1 << 38, cudaSuccess; }
+cudaError_t cudaMemPoolCreate(cudaMemPool_t* p, const cudaMemPoolProps*) { return fake::handle(p); }
+cudaError_t cudaMemPoolSetAttribute(cudaMemPool_t, cudaMemPoolAttr, void*) { return cudaSuccess; }
+cudaError_t cudaMemPoolDestroy(cudaMemPool_t) { return cudaSuccess; }
+cudaError_t cudaMallocFromPoolAsync(void** p, size_t n, cudaMemPool_t, cudaStream_t) { return fake::alloc(p, n); }
+cudaError_t cudaFreeAsync(void* p, cudaStream_t) { return fake::release(p); }
+cudaError_t cudaEventQuery(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaMemsetAsync(void* p, int, size_t, cudaStream_t) { return fake::null_copies += !p, cudaSuccess; }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) { return fake::handle(s); }
 cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }

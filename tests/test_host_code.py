@@ -10,7 +10,7 @@ from broxy_gb300 import _lib as L
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
-@pytest.mark.parametrize("tu", ["test_launch_status.cpp", "test_batch_graph.cpp", "test_batch_alloc.cpp", "test_frame_field_alloc.cpp"])
+@pytest.mark.parametrize("tu", ["test_launch_status.cpp", "test_batch_graph.cpp", "test_batch_alloc.cpp", "test_frame_field_alloc.cpp", "test_stale_error.cpp"])
 def test_host_code(tmp_path, tu):
     from __graft_entry__ import build
     build()
